@@ -205,16 +205,27 @@ __device__ __forceinline__ void sweep_dw(const float2 (&In)[TZ + 2][RX + 2], flo
 //  * x-box: the squares are folded into the first additions as FMAs
 //    (g = d0*d0 + (d1*d1 + d2*d2) with the inner pair shared by two outputs), 6 instructions per
 //    plane of 3 outputs instead of 5 multiplies + 5 adds.
+//    The three additions are m = S.x + S.y and one packed (m, m) + (left, right): what bounds the
+//    loop is the issue of operands, and a packed instruction with at most two distinct operand
+//    pairs costs the same two cycles as two scalar ones but loads the two halves of the FMA pipe
+//    equally (scalar additions pile up on one half: 72.6 % against 61.8 % busy). With the shared
+//    loads visible to the compiler and the warp index known to be uniform, NH 11 at 222x222x112,
+//    10 atlases takes 28.4 ms (29.2 ms before; 1965 MHz).
 //  * labels ride a register ring like the atlas planes: one new plane per dw step.
 //  * a pair's shared-memory address is 8-byte aligned for every other dv (the parity of
 //    dv + HW): those sweeps load pairs with one 64-bit LDS, the others with two 32-bit LDS.
 
+// (plain loads, not volatile asm: the compiler may then move them across the arithmetic)
+__device__ __forceinline__ float shared_f32(uint32_t addr) {
+  return *static_cast<const float *>(__cvta_shared_to_generic(addr));
+}
+
 template <bool AL>
 __device__ __forceinline__ float2 lds_pair(uint32_t addr) {
   if constexpr (AL) {
-    return lds_f32x2(addr);
+    return *static_cast<const float2 *>(__cvta_shared_to_generic(addr));
   } else {
-    return make_float2(lds_f32(addr), lds_f32(addr + 4));
+    return make_float2(shared_f32(addr), shared_f32(addr + 4));
   }
 }
 
@@ -310,7 +321,8 @@ __device__ __forceinline__ void sweep_dw_yp(const float2 (&In)[TZ + 2][RX + 2],
             const float lft = __shfl_up_sync(0xffffffffu, cc.y, 1, 16);
             const float rgt = __shfl_down_sync(0xffffffffu, cc.x, 1, 16);
             const float m = cc.x + cc.y;
-            const float2 w = make_float2(ex2_approx(-(m + lft)), ex2_approx(-(m + rgt)));
+            const float2 e = add2(make_float2(m, m), make_float2(lft, rgt));
+            const float2 w = make_float2(ex2_approx(-e.x), ex2_approx(-e.y));
             const float2 lab = LR ? Lw[(q + k + jj) % NQ][x]
                                   : lds_pair<AL>(rowL[x] + so + (q + k) * C::PLANE);
             P[q + k][x] = fma2(w, lab, P[q + k][x]);
@@ -341,7 +353,9 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
   const uint32_t bar0 = pp.base, bar1 = pp.base + 8;
   const uint32_t ringA = pp.base + 128;
   const uint32_t ringL = ringA + C::RA * C::SLOT_A;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // (the shuffle tells the compiler that the warp index, and every ring address made from it, is
+  // uniform over the warp)
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lo = HW + 1;
   const float2 scale2 = make_float2(sv.scale, sv.scale);
   int grp, t, a_first, natl;
@@ -607,9 +621,18 @@ template <> struct TileOf<2, 2> { static constexpr int RX = 3, TZ = 3, LY = 0, M
 template <int HW> struct TileOf<3, HW> { static constexpr int RX = 3, TZ = 4, LY = 2, MB = 1; };
 template <> struct TileOf<3, 1> { static constexpr int RX = 4, TZ = 2, LY = 2, MB = 1; };
 template <int HW> struct TileOf<4, HW> { static constexpr int RX = 2, TZ = 3, LY = 1, MB = 3; };
+// The batched kernel's tiles: one kernel holds the tile code of three windows beside the walk over
+// the subject table, and the register tiles that fill 255 registers by themselves spill there (500
+// bytes of spill loads with set 0's). Set 0 takes y-pairs (2,4): 250 registers, no spills. Six
+// subjects of 64..160 x 64..160 x 48..96, 2..8 atlases, NH 7/9/11: 7.73 ms against 8.73; (2,5) for
+// NH 11 7.83, (2,6) 7.87; sixteen such subjects 24.6 ms against 28.6.
+template <int SET, int HW> struct BatchTileOf : TileOf<SET, HW> {};
+template <> struct BatchTileOf<0, 5> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
+template <> struct BatchTileOf<0, 4> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
+template <> struct BatchTileOf<0, 3> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
 template <int SET, int HW>
 constexpr int smem_of() {
-  return Cfg<HW, TileOf<SET, HW>::RX, TileOf<SET, HW>::TZ>::SMEM;
+  return Cfg<HW, BatchTileOf<SET, HW>::RX, BatchTileOf<SET, HW>::TZ>::SMEM;
 }
 template <int SET>
 constexpr int batch_smem() {
@@ -630,7 +653,7 @@ struct BatchParams {
 // items of all subjects are numbered consecutively; each CTA walks the list with a grid stride
 // and dispatches every item to the tile code of its subject's window.
 template <int SET>
-__global__ void __launch_bounds__(kThreads, TileOf<SET, 5>::MB) fuse_batch_kernel(const BatchParams bp) {
+__global__ void __launch_bounds__(kThreads, BatchTileOf<SET, 5>::MB) fuse_batch_kernel(const BatchParams bp) {
   extern __shared__ unsigned char smem_raw[];
   // The current subject's view, copied into shared memory when the subject changes: the tile
   // code then reads its fields from there as it needs them instead of keeping the values it
@@ -654,9 +677,9 @@ __global__ void __launch_bounds__(kThreads, TileOf<SET, 5>::MB) fuse_batch_kerne
     const int local = item - sv.item_begin;
     bool ok = true;
     switch (sv.hw) {
-      case 5: ok = run_item<5, TileOf<SET, 5>::RX, TileOf<SET, 5>::TZ, TileOf<SET, 5>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
-      case 4: ok = run_item<4, TileOf<SET, 4>::RX, TileOf<SET, 4>::TZ, TileOf<SET, 4>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
-      default: ok = run_item<3, TileOf<SET, 3>::RX, TileOf<SET, 3>::TZ, TileOf<SET, 3>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
+      case 5: ok = run_item<5, BatchTileOf<SET, 5>::RX, BatchTileOf<SET, 5>::TZ, BatchTileOf<SET, 5>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
+      case 4: ok = run_item<4, BatchTileOf<SET, 4>::RX, BatchTileOf<SET, 4>::TZ, BatchTileOf<SET, 4>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
+      default: ok = run_item<3, BatchTileOf<SET, 3>::RX, BatchTileOf<SET, 3>::TZ, BatchTileOf<SET, 3>::LY>(sv, local, pp, bp.err, bp.timeout_ns, -1); break;
     }
     if (!ok) {
       pipe_drain(pp, bp.timeout_ns);
@@ -775,6 +798,17 @@ struct Plan {
   int blocks, groups, ntiles, tiles_y, tiles_x, tiles_z, rx, tz;
 };
 
+template <class T, int HW>
+void tile_counts(const Geometry &g, Plan *pl) {
+  constexpr int XC = Cfg<HW, T::RX, T::TZ>::XC;
+  pl->rx = T::RX;
+  pl->tz = T::TZ;
+  pl->tiles_y = (g.iy + kOutY - 1) / kOutY;
+  pl->tiles_x = (g.ix + XC - 1) / XC;
+  pl->tiles_z = (g.iz + 2 * T::TZ - 1) / (2 * T::TZ);
+  pl->ntiles = pl->tiles_y * pl->tiles_x * pl->tiles_z;
+}
+
 template <int SET, int HW>
 cudaError_t plan_hw(const Geometry &g, Plan *pl) {
   constexpr int RX = TileOf<SET, HW>::RX, TZ = TileOf<SET, HW>::TZ, LY = TileOf<SET, HW>::LY;
@@ -789,12 +823,7 @@ cudaError_t plan_hw(const Geometry &g, Plan *pl) {
       cudaSuccess)
     return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-  pl->rx = RX;
-  pl->tz = TZ;
-  pl->tiles_y = (g.iy + kOutY - 1) / kOutY;
-  pl->tiles_x = (g.ix + C::XC - 1) / C::XC;
-  pl->tiles_z = (g.iz + 2 * TZ - 1) / (2 * TZ);
-  pl->ntiles = pl->tiles_y * pl->tiles_x * pl->tiles_z;
+  tile_counts<TileOf<SET, HW>, HW>(g, pl);
   const int slots = sm_count() * per_sm;
   pl->groups = choose_groups(pl->ntiles, g.num, slots);
   const long long items = (long long)pl->ntiles * pl->groups;
@@ -905,10 +934,12 @@ cudaError_t launch_set(const Geometry &g, const SlabInputs &in, float *out, doub
   }
 }
 
-// Slab box sizes of one subject under a tile set (for its tensor maps in the batch).
+// Tiles and slab box sizes of one subject in the batched kernel.
 template <int SET, int HW>
-void boxes_hw(int *yb, int *za, int *zl) {
-  using C = Cfg<HW, TileOf<SET, HW>::RX, TileOf<SET, HW>::TZ>;
+void batch_plan_hw(const Geometry &g, Plan *pl, int *yb, int *za, int *zl) {
+  using T = BatchTileOf<SET, HW>;
+  using C = Cfg<HW, T::RX, T::TZ>;
+  tile_counts<T, HW>(g, pl);
   *yb = C::YB;
   *za = C::ZA;
   *zl = C::ZL;
@@ -916,14 +947,13 @@ void boxes_hw(int *yb, int *za, int *zl) {
 
 template <int SET>
 cudaError_t batch_plan(int hw, const Geometry &g, Plan *pl, int *yb, int *za, int *zl) {
-  cudaError_t e;
+  *pl = Plan{};
   switch (hw) {
-    case 5: e = plan_hw<SET, 5>(g, pl); boxes_hw<SET, 5>(yb, za, zl); break;
-    case 4: e = plan_hw<SET, 4>(g, pl); boxes_hw<SET, 4>(yb, za, zl); break;
-    case 3: e = plan_hw<SET, 3>(g, pl); boxes_hw<SET, 3>(yb, za, zl); break;
+    case 5: batch_plan_hw<SET, 5>(g, pl, yb, za, zl); return cudaSuccess;
+    case 4: batch_plan_hw<SET, 4>(g, pl, yb, za, zl); return cudaSuccess;
+    case 3: batch_plan_hw<SET, 3>(g, pl, yb, za, zl); return cudaSuccess;
     default: return cudaErrorInvalidValue;
   }
-  return e;
 }
 
 template <int SET>
