@@ -148,14 +148,38 @@ int select_device(pct_handle *h) {
 
 constexpr size_t kMaxTimedLaunches = 4096;  // pct_set_kernel_timing: pairs kept between reads
 
+// Plans the plain kernel and makes room for its partial sums. The plan keeps to what the handle's
+// memory cap leaves for them once its other buffers have grown by `others_grow` bytes, and to what
+// is there already when the stream is being captured (no allocation then) or the device has no
+// more: one group needs none, so a plan always exists.
+int plan_fusion(pct_handle *h, const pct::Geometry &g, size_t others_grow, cudaStream_t s,
+                pct::FusePlan *plan) {
+  size_t limit = SIZE_MAX;
+  if (h->mem_limit) {
+    const size_t others = h->allocated - h->partial.bytes + others_grow;
+    limit = h->mem_limit > others ? h->mem_limit - others : 0;
+  }
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
+    cudaGetLastError();  // (a legacy default stream while another one is captured)
+    capturing = cudaStreamCaptureStatusActive;
+  }
+  if (capturing != cudaStreamCaptureStatusNone) limit = std::min(limit, h->partial.bytes);
+  PCT_CUDA(h, pct::fuse_tma_plan(g, h->tile_set, limit, plan));
+  if (!plan->partial_bytes || !ensure(h, h->partial, plan->partial_bytes)) return PCT_OK;
+  h->last_error.clear();
+  PCT_CUDA(h, pct::fuse_tma_plan(g, h->tile_set, h->partial.bytes, plan));
+  return PCT_OK;
+}
+
 // Zeroes the device status word and enqueues the TMA-staged fusion kernel.
 int launch_fusion(pct_handle *h, const pct::Geometry &g, const pct::SlabInputs &in, float *d_out,
                   double div, cudaStream_t s) {
   int st = ensure(h, h->err, 16);
   if (st) return st;
   int *err = static_cast<int *>(h->err.ptr);
-  const size_t pbytes = pct::fuse_tma_partial_bytes(g, h->tile_set);
-  if (pbytes && (st = ensure(h, h->partial, pbytes))) return st;
+  pct::FusePlan plan;
+  if ((st = plan_fusion(h, g, 0, s, &plan))) return st;
   PCT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), s));
   pct::LaunchHooks wt{h->wait_test_ns, nullptr, nullptr};
   h->wait_test_ns = 0;
@@ -170,7 +194,7 @@ int launch_fusion(pct_handle *h, const pct::Geometry &g, const pct::SlabInputs &
     wt.stop = h->kt_ev[2 * h->kt_used + 1];
   }
   PCT_CUDA(h, pct::launch_fuse_tma(g, in, d_out, div, static_cast<float *>(h->partial.ptr), err, wt,
-                                   h->tile_set, s));
+                                   plan, s));
   if (wt.stop) ++h->kt_used;  // a pair is read only once the launch between its events was enqueued
   return PCT_OK;
 }
@@ -369,15 +393,20 @@ int stage_pitched_slice(pct_handle *h, DevBuf &buf, float *stage_base, const flo
 int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, const float *atlas,
                    const float *atlas_ct, float *d_out, double div, bool normalize,
                    float *host_out, cudaStream_t s) {
-  pct::FusePlanInfo pl;
-  PCT_CUDA(h, pct::fuse_tma_plan(g, h->tile_set, &pl));
-  if (pl.groups < 2 || h->wait_test_ns) return PCT_ERR_UNSUPPORTED;
   const int pitch = pct::slab_pitch(g.ny);
   const size_t rows = (size_t)g.num * g.nz * g.nx;
-  int st;
+  auto grow = [](const DevBuf &b, size_t bytes) { return bytes > b.bytes ? bytes - b.bytes : 0; };
+  pct::FusePlan pl;
+  // (room for the one-upload path's staging stack too, which a cap may leave instead of two)
+  int st = plan_fusion(h, g,
+                       grow(h->atlas, rows * pitch * sizeof(float)) +
+                           grow(h->label, rows * pitch * sizeof(float)) + grow(h->err, 16) +
+                           (pitch != g.ny ? grow(h->stage, rows * g.ny * sizeof(float)) : 0),
+                       s, &pl);
+  if (st) return st;
+  if (pl.atlas_groups < 2 || h->wait_test_ns) return PCT_ERR_UNSUPPORTED;
   if ((st = ensure(h, h->atlas, rows * pitch * sizeof(float))) ||
-      (st = ensure(h, h->label, rows * pitch * sizeof(float))) ||
-      (st = ensure(h, h->partial, pl.partial_bytes)) || (st = ensure(h, h->err, 16)))
+      (st = ensure(h, h->label, rows * pitch * sizeof(float))) || (st = ensure(h, h->err, 16)))
     return st;
   if (pitch != g.ny && ensure(h, h->stage, 2 * rows * g.ny * sizeof(float))) {
     h->last_error.clear();  // over the handle's memory cap: the one-upload path needs half
@@ -390,11 +419,19 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     int o0, o1;          // output planes to combine and download after it (none when o0 == o1)
   };
   std::vector<Part> parts;
-  const int per = g.num / pl.groups;
+  const int per = g.num / pl.atlas_groups;
   // z-tile tz holds the output planes [lo + 2 tz TZ, lo + 2 tz TZ + 2 TZ)
   auto out_plane = [&](int tz) { return tz >= pl.tiles_z ? g.nz : g.lo + 2 * pl.tz * tz; };
-  const int first = std::min(pl.tiles_z, (pl.ctas + pl.tiles_xy - 1) / pl.tiles_xy);
-  {
+  const int tiles_xy = pl.tiles_x * pl.tiles_y;
+  const int first = std::min(pl.tiles_z, (pl.ctas + tiles_xy - 1) / tiles_xy);
+  if (pl.splits > 1) {  // a small volume: one part per atlas group, its items for the whole window
+    const int items = pl.splits * pl.tiles;
+    for (int grp = 0; grp < pl.atlas_groups; ++grp) {
+      const bool out_now = host_out && grp == pl.atlas_groups - 1;
+      parts.push_back(Part{grp == 0, grp * per, (grp + 1) * per, 0, g.nz, grp * items,
+                           (grp + 1) * items, 0, out_now ? g.nz : 0});
+    }
+  } else {
     // z-tile ends of the first group's leading parts; part k reads planes [0, planes_read(end))
     const int ends[2] = {first, std::min(pl.tiles_z, 2 * first)};
     int z0 = 0, t0 = 0;
@@ -402,11 +439,11 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
       if (e <= t0 || e >= pl.tiles_z) continue;
       const int z1 = pct::fuse_tma_planes_read(g, pl, e);
       if (z1 >= g.nz) continue;
-      parts.push_back(Part{true, 0, per, z0, z1, t0 * pl.tiles_xy, e * pl.tiles_xy, 0, 0});
+      parts.push_back(Part{true, 0, per, z0, z1, t0 * tiles_xy, e * tiles_xy, 0, 0});
       z0 = z1;
       t0 = e;
     }
-    parts.push_back(Part{true, 0, per, z0, g.nz, t0 * pl.tiles_xy, pl.tiles, 0, 0});
+    parts.push_back(Part{true, 0, per, z0, g.nz, t0 * tiles_xy, pl.tiles, 0, 0});
     for (int grp = 1; grp < pl.groups - 1; ++grp)
       parts.push_back(Part{false, grp * per, (grp + 1) * per, 0, g.nz, grp * pl.tiles,
                            (grp + 1) * pl.tiles, 0, 0});
@@ -424,7 +461,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
         const int t0 = starts[k], t1 = k < 2 ? starts[k + 1] : pl.tiles_z;
         if (t1 <= t0) continue;
         parts.push_back(Part{false, last * per, g.num, 0, uploaded ? 0 : g.nz,
-                             base + t0 * pl.tiles_xy, base + t1 * pl.tiles_xy,
+                             base + t0 * tiles_xy, base + t1 * tiles_xy,
                              t0 == 0 ? 0 : out_plane(t0), out_plane(t1)});
         uploaded = true;
       }
@@ -486,7 +523,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     }
     const cudaStream_t ls = lanes[k & 1];
     PCT_CUDA(h, cudaStreamWaitEvent(ls, landed(last_upload), 0));
-    PCT_CUDA(h, pct::launch_fuse_tma_items(g, in, div, partial, err, h->tile_set, p.i0, p.i1, ls));
+    PCT_CUDA(h, pct::launch_fuse_tma_items(g, in, div, partial, err, pl, p.i0, p.i1, ls));
     PCT_CUDA(h, cudaEventRecord(done(k), ls));
     return PCT_OK;
   };
@@ -497,7 +534,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     const Part &p = parts[k];
     PCT_CUDA(h, cudaStreamWaitEvent(os, done(k), 0));
     PCT_CUDA(h, cudaStreamWaitEvent(os, done(k - 1), 0));
-    PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, h->tile_set, d_out, p.o0, p.o1, os));
+    PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, p.o0, p.o1, os));
     PCT_CUDA(h, cudaMemcpyAsync(host_out + p.o0 * plane, d_out + p.o0 * plane,
                                 (size_t)(p.o1 - p.o0) * plane * sizeof(float),
                                 cudaMemcpyDeviceToHost, os));
@@ -522,7 +559,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
   }
   if (st) return st;
   if (!host_out)
-    PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, h->tile_set, d_out, 0, g.nz, s));
+    PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, 0, g.nz, s));
   return PCT_OK;
 }
 
@@ -939,8 +976,8 @@ int pct_query_plan(int device, int nx, int ny, int nz, int num_atlas, int nh, pc
   int prev = 0;
   cudaGetDevice(&prev);
   if (cudaSetDevice(device) != cudaSuccess) return PCT_ERR_NO_DEVICE;
-  pct::FusePlanInfo info;
-  const cudaError_t e = pct::fuse_tma_plan(g, 0, &info);
+  pct::FusePlan info;
+  const cudaError_t e = pct::fuse_tma_plan(g, 0, SIZE_MAX, &info);
   cudaSetDevice(prev);
   if (e != cudaSuccess) {
     cudaGetLastError();

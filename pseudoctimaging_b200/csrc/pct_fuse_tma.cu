@@ -94,6 +94,7 @@ struct SubjectView {
   float scale;        // sqrt(log2(e)/div): taps are scaled so that the box sum is SSD*log2(e)/div
   int tiles_y, tiles_x, ntiles;
   int groups, atlases_per_group;  // items = groups * ntiles (group-major)
+  int splits;         // groups per atlas group: each takes a range of the window's x offsets
   int hw;             // half window of this subject (batched kernel dispatch)
   int item_begin;     // first global item of this subject (batched kernel)
   int atlas_base;     // first atlas of group 0 (a single-atlas launch over a tile list)
@@ -359,6 +360,7 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
   const int lo = HW + 1;
   const float2 scale2 = make_float2(sv.scale, sv.scale);
   int grp, t, a_first, natl;
+  int j0 = 0, nj = NS;  // the item's x offsets du = j - HW, j in [j0, j0 + nj)
   uint32_t later = 0;  // masked items: the pair's atlases after the current one (bits)
   if constexpr (MASKED) {
     grp = (int)((uint32_t)item >> 24);
@@ -371,10 +373,13 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
   } else {
     grp = item / sv.ntiles;
     t = item - grp * sv.ntiles;
-    a_first = sv.atlas_base + grp * sv.atlases_per_group;
+    const int ag = grp / sv.splits, part = grp - ag * sv.splits;
+    a_first = sv.atlas_base + ag * sv.atlases_per_group;
     natl = sv.atlases_per_group;
+    j0 = part * NS / sv.splits;
+    nj = (part + 1) * NS / sv.splits - j0;
   }
-  const int T = natl * NS;  // du steps per item (atlas-major)
+  const int T = natl * nj;  // du steps per item (atlas-major)
   const int ty = t % sv.tiles_y;
   t /= sv.tiles_y;
   const int txc = t % sv.tiles_x;
@@ -421,7 +426,7 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
 
   int a = a_first;
   for (int i = 0; i < T; ++i, ++pp.gstep) {
-    const int ai = i / NS, j = i - ai * NS;
+    const int ai = i / nj, j = j0 + i - ai * nj;
     if constexpr (MASKED) {
       if (j == 0 && i > 0) {  // the pair's second atlas
         a = sv.atlas_base + __ffs(later) - 1;
@@ -437,16 +442,16 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
       fence_proxy_async_smem();
       // Testing hook: withhold the first window of this CTA so that the wait below runs out.
       const bool withhold = (int)blockIdx.x == withhold_cta && gstep == 0;
-      if (j == 0 && !withhold) {  // atlas start: the whole window for this step
+      if (j == j0 && !withhold) {  // atlas start: the whole window for this step
         const uint32_t b = (gstep & 1) ? bar1 : bar0;
         mbar_arrive_expect_tx(b, (C::XC + 2) * C::ROW_A + C::XC * C::ROW_L);
-        for (int k = 0; k < C::XC + 2; ++k)
+        for (int k = j; k < j + C::XC + 2; ++k)
           tma_load_4d(ringA + (k % C::RA) * C::SLOT_A, sv.tmA, b, ybox, xA + k, zA, a);
-        for (int k = 0; k < C::XC; ++k)
+        for (int k = j; k < j + C::XC; ++k)
           tma_load_4d(ringL + (k % C::RL) * C::SLOT_L, sv.tmL, b, ybox, xL + k, zL, a);
       }
       pp.armed_next = false;
-      if (j + 1 < NS) {  // prefetch the one new row of each ring for step i+1
+      if (j + 1 < j0 + nj) {  // prefetch the one new row of each ring for step i+1
         const uint32_t b = ((gstep + 1) & 1) ? bar1 : bar0;
         mbar_arrive_expect_tx(b, C::ROW_A + C::ROW_L);
         const int ka = j + C::XC + 2, kl = j + C::XC;
@@ -621,15 +626,19 @@ template <> struct TileOf<2, 2> { static constexpr int RX = 3, TZ = 3, LY = 0, M
 template <int HW> struct TileOf<3, HW> { static constexpr int RX = 3, TZ = 4, LY = 2, MB = 1; };
 template <> struct TileOf<3, 1> { static constexpr int RX = 4, TZ = 2, LY = 2, MB = 1; };
 template <int HW> struct TileOf<4, HW> { static constexpr int RX = 2, TZ = 3, LY = 1, MB = 3; };
+// Further y-pair tiles, which set 0 of the single-subject kernel chooses between by the volume's
+// shape (kTileCost): (2,5), (2,6) and (2,4).
+template <int HW> struct TileOf<5, HW> { static constexpr int RX = 2, TZ = 5, LY = 1, MB = 1; };
+template <int HW> struct TileOf<6, HW> { static constexpr int RX = 2, TZ = 6, LY = 1, MB = 1; };
+template <int HW> struct TileOf<7, HW> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
+
 // The batched kernel's tiles: one kernel holds the tile code of three windows beside the walk over
 // the subject table, and the register tiles that fill 255 registers by themselves spill there (500
 // bytes of spill loads with set 0's). Set 0 takes y-pairs (2,4): 250 registers, no spills. Six
 // subjects of 64..160 x 64..160 x 48..96, 2..8 atlases, NH 7/9/11: 7.73 ms against 8.73; (2,5) for
 // NH 11 7.83, (2,6) 7.87; sixteen such subjects 24.6 ms against 28.6.
 template <int SET, int HW> struct BatchTileOf : TileOf<SET, HW> {};
-template <> struct BatchTileOf<0, 5> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
-template <> struct BatchTileOf<0, 4> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
-template <> struct BatchTileOf<0, 3> { static constexpr int RX = 2, TZ = 4, LY = 1, MB = 1; };
+template <int HW> struct BatchTileOf<0, HW> : TileOf<7, HW> {};
 template <int SET, int HW>
 constexpr int smem_of() {
   return Cfg<HW, BatchTileOf<SET, HW>::RX, BatchTileOf<SET, HW>::TZ>::SMEM;
@@ -769,24 +778,6 @@ cudaError_t launch_combine_groups(const Geometry &g, const float *partial, int g
   return launch_combine_groups(g, partial, groups, out, 0, g.nz, stream);
 }
 
-// Picks the number of atlas groups (a divisor of num) so that the work items fill the
-// persistent grid's rounds: the first group count reaching 97% round occupancy, else the best.
-int choose_groups(int ntiles, int num, int slots) {
-  int best = 1;
-  double best_eff = 0.0;
-  for (int g = 1; g <= num; ++g) {
-    if (num % g) continue;
-    const double rounds = (double)ntiles * g / slots;
-    const double eff = rounds / std::ceil(rounds);
-    if (eff >= 0.97) return g;
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = g;
-    }
-  }
-  return best;
-}
-
 int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -794,45 +785,115 @@ int sm_count() {
   return sms;
 }
 
-struct Plan {
-  int blocks, groups, ntiles, tiles_y, tiles_x, tiles_z, rx, tz;
-};
-
 template <class T, int HW>
-void tile_counts(const Geometry &g, Plan *pl) {
+void tile_counts(const Geometry &g, FusePlan *pl) {
   constexpr int XC = Cfg<HW, T::RX, T::TZ>::XC;
   pl->rx = T::RX;
   pl->tz = T::TZ;
   pl->tiles_y = (g.iy + kOutY - 1) / kOutY;
   pl->tiles_x = (g.ix + XC - 1) / XC;
   pl->tiles_z = (g.iz + 2 * T::TZ - 1) / (2 * T::TZ);
-  pl->ntiles = pl->tiles_y * pl->tiles_x * pl->tiles_z;
+  pl->tiles = pl->tiles_y * pl->tiles_x * pl->tiles_z;
+}
+
+// Measured cost of one output voxel of a tile, padding included, for all NH^3 offsets of one atlas
+// (ns of the whole chip; 222x222x112, 10 atlases, two CTAs per SM), by half window and tile: (3,4) (NH 9: (3,3)
+// with the label ring, NH 5: (3,3), NH 3: (4,2)), (2,5), (2,6), (2,4). Within a few per cent of
+// each other, so that what decides is how much of the volume's last tiles is padding (NH 11 at
+// 222x222x112: (2,5) tiles the 210 x 210 x 100 interior with 4 % less of it than (3,4)).
+constexpr int kTileChoices[4] = {0, 5, 6, 7};
+constexpr float kTileCost[5][4] = {{0.0185f, 0.0162f, 0.0146f, 0.0195f},
+                                   {0.0635f, 0.0642f, 0.0643f, 0.0629f},
+                                   {0.1708f, 0.1625f, 0.1575f, 0.1685f},
+                                   {0.3510f, 0.3376f, 0.3356f, 0.3344f},
+                                   {0.6020f, 0.5990f, 0.5970f, 0.6080f}};
+
+// Expected time (us) of the volume's work items, `natl` atlases and 1 / splits of the window each:
+// rounds of the persistent grid, the last one cheaper when it leaves SMs with one CTA (one warp per
+// scheduler takes 0.61 of the time of two sharing it; 0.85 measured behind a full round), plus what
+// each item spends on its windows, taps and stores and, with partial sums, the combine. Within 10 %
+// of the measured times for 17 shapes from 48x40x30 to 222x222x112, every tile and split; the plan
+// chosen is 0..2 % behind the best of them on 14 of the 17, 11 % at worst.
+double expected_us(const Geometry &g, const FusePlan &pl, int slots, double voxel_ns, int natl,
+                   int splits, int groups) {
+  const double rounds = (double)pl.tiles * groups / slots;
+  const double full = std::floor(rounds), rem = rounds - full;
+  const double voxels = (double)kOutY * kWarps * pl.rx * 2 * pl.tz;
+  const double round = 1e-3 * slots * voxels * voxel_ns * natl / splits;  // items of average length
+  const double longest = round * splits * ((g.nh + splits - 1) / splits) / g.nh;
+  double t = 0.0;
+  if (full < 1.0)
+    t = (rem <= 0.5 ? 0.61 : 1.0) * longest;
+  else if (rem > 0.0)
+    t = std::min((full + (rem <= 0.5 ? 0.85 : 1.0)) * round, (rounds + 0.4) * round) + longest - round;
+  else
+    t = full * round + longest - round;
+  t += std::max(1.0, rounds) * (6.0 + 1.0 * natl);
+  if (groups > 1) t += 2.5 + (double)g.ix * g.iy * g.iz * 16.0 * groups / 5e6;
+  return t;
+}
+
+// Chooses the atlas groups and, once every atlas is a group of its own, the ranges of the window's
+// rows that the items of a tile are split into, for one tile shape: fills *pl and returns its
+// expected time. Small volumes have fewer tiles than the chip has room for (64x64x32, one atlas:
+// 42 tiles on 148 SMs, 81 us for one CTA's 343 offsets), so their windows are split over CTAs.
+// Three groups or more are taken over fewer when they cost at most 3 % more: the host-pointer path
+// overlaps its uploads with the fusion group by group, and the FP32 sums are shorter.
+double choose_groups(const Geometry &g, int slots, double voxel_ns, size_t partial_limit,
+                     FusePlan *pl) {
+  const int ns = g.nh;
+  auto bytes_of = [&](int groups) {
+    return groups > 1 ? (size_t)groups * 2 * (size_t)g.nvox() * sizeof(float) : 0;
+  };
+  auto time_of = [&](int agroups, int splits) {
+    const int groups = agroups * splits;
+    if (bytes_of(groups) > partial_limit || (long long)pl->tiles * groups >= (1LL << 31)) return -1.0;
+    return expected_us(g, *pl, slots, voxel_ns, g.num / agroups, splits, groups);
+  };
+  int agroups = 1, splits = 1;
+  double best = time_of(1, 1);
+  auto consider = [&](int a, int sp) {
+    const double t = time_of(a, sp);
+    if (t < 0.0 || t >= best) return;
+    best = t;
+    agroups = a;
+    splits = sp;
+  };
+  for (int a = 2; a <= g.num; ++a)
+    if (g.num % a == 0) consider(a, 1);
+  for (int sp = 2; sp <= ns; ++sp) consider(g.num, sp);
+  if (splits == 1 && agroups < 3)
+    for (int a = 3; a <= g.num; ++a) {
+      if (g.num % a) continue;
+      const double t = time_of(a, 1);
+      if (t < 0.0 || t > 1.03 * best) continue;
+      best = t;
+      agroups = a;
+      break;
+    }
+  pl->atlas_groups = agroups;
+  pl->splits = splits;
+  pl->groups = agroups * splits;
+  pl->partial_bytes = bytes_of(pl->groups);
+  return best;
 }
 
 template <int SET, int HW>
-cudaError_t plan_hw(const Geometry &g, Plan *pl) {
-  constexpr int RX = TileOf<SET, HW>::RX, TZ = TileOf<SET, HW>::TZ, LY = TileOf<SET, HW>::LY;
-  using C = Cfg<HW, RX, TZ>;
-  auto kern = fuse_tma_kernel<HW, RX, TZ, LY, TileOf<SET, HW>::MB>;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)) !=
-      cudaSuccess)
-    return e;
-  int per_sm = 1;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, C::SMEM)) !=
-      cudaSuccess)
-    return e;
-  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-  tile_counts<TileOf<SET, HW>, HW>(g, pl);
-  const int slots = sm_count() * per_sm;
-  pl->groups = choose_groups(pl->ntiles, g.num, slots);
-  const long long items = (long long)pl->ntiles * pl->groups;
-  pl->blocks = (int)(items < slots ? items : slots);
-  return cudaSuccess;
+double plan_hw(const Geometry &g, int sms, double voxel_ns, size_t partial_limit, FusePlan *pl) {
+  using T = TileOf<SET, HW>;
+  // two CTAs share an SM's shared memory (228 KB, 1 KB reserved per CTA) and registers
+  static_assert(T::MB > 1 || 2 * (Cfg<HW, T::RX, T::TZ>::SMEM + 1024) <= 228 * 1024, "2 CTAs per SM");
+  tile_counts<T, HW>(g, pl);
+  pl->set = SET;
+  const int slots = sms * (T::MB > 1 ? T::MB : 2);
+  const double t = choose_groups(g, slots, voxel_ns, partial_limit, pl);
+  const long long items = (long long)pl->tiles * pl->groups;
+  pl->ctas = (int)(items < slots ? items : slots);
+  return t;
 }
 
 SubjectView subject_view(const Geometry &g, const SlabInputs &in, float *out, double div,
-                         float *partial, const Plan &pl) {
+                         float *partial, const FusePlan &pl) {
   SubjectView sv{};
   sv.img = in.img;
   sv.out = out;
@@ -845,30 +906,33 @@ SubjectView subject_view(const Geometry &g, const SlabInputs &in, float *out, do
   sv.scale = (float)sqrt(1.4426950408889634 / div);
   sv.tiles_y = pl.tiles_y;
   sv.tiles_x = pl.tiles_x;
-  sv.ntiles = pl.ntiles;
+  sv.ntiles = pl.tiles;
   sv.groups = pl.groups;
-  sv.atlases_per_group = g.num / pl.groups;
+  sv.splits = pl.splits;
+  sv.atlases_per_group = g.num / pl.atlas_groups;
   sv.hw = g.hw;
   return sv;
 }
 
 template <int SET, int HW>
 cudaError_t launch_hw(const Geometry &g, const SlabInputs &in, float *out, double div,
-                      float *partial, int *err, const LaunchHooks &wt, int item_begin, int item_end,
-                      cudaStream_t stream) {
-  constexpr int RX = TileOf<SET, HW>::RX, TZ = TileOf<SET, HW>::TZ;
-  using C = Cfg<HW, RX, TZ>;
-  Plan pl;
-  cudaError_t e = plan_hw<SET, HW>(g, &pl);
-  if (e != cudaSuccess) return e;
+                      float *partial, int *err, const LaunchHooks &wt, const FusePlan &pl,
+                      int item_begin, int item_end, cudaStream_t stream) {
+  using T = TileOf<SET, HW>;
+  using C = Cfg<HW, T::RX, T::TZ>;
   if (pl.groups > 1 && !partial) return cudaErrorInvalidValue;
   const bool whole = item_begin < 0;  // every item, then the combine
   if (whole) {
     item_begin = 0;
-    item_end = pl.groups * pl.ntiles;
-  } else if (pl.groups < 2 || item_begin >= item_end || item_end > pl.groups * pl.ntiles) {
+    item_end = pl.groups * pl.tiles;
+  } else if (pl.groups < 2 || item_begin >= item_end || item_end > pl.groups * pl.tiles) {
     return cudaErrorInvalidValue;  // an item range needs partial sums and a later combine
   }
+  auto kern = fuse_tma_kernel<HW, T::RX, T::TZ, T::LY, T::MB>;
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)) !=
+      cudaSuccess)
+    return e;
   CUtensorMap tmA, tmL;
   if ((e = make_slab_map(&tmA, in.atlas, g.nx, g.ny, g.nz, g.num, in.pitch, C::YB, C::ZA)) !=
       cudaSuccess)
@@ -887,10 +951,9 @@ cudaError_t launch_hw(const Geometry &g, const SlabInputs &in, float *out, doubl
   }
   p.item_begin = item_begin;
   p.item_end = item_end;
-  const int blocks = std::min(pl.blocks, p.item_end - p.item_begin);
+  const int blocks = std::min(pl.ctas, p.item_end - p.item_begin);
   if (wt.start && (e = cudaEventRecord(wt.start, stream)) != cudaSuccess) return e;
-  fuse_tma_kernel<HW, RX, TZ, TileOf<SET, HW>::LY, TileOf<SET, HW>::MB>
-      <<<blocks, kThreads, C::SMEM, stream>>>(tmA, tmL, p);
+  kern<<<blocks, kThreads, C::SMEM, stream>>>(tmA, tmL, p);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (wt.stop && (e = cudaEventRecord(wt.stop, stream)) != cudaSuccess) return e;
   if (whole && pl.groups > 1) return launch_combine_groups(g, partial, pl.groups, out, stream);
@@ -898,45 +961,63 @@ cudaError_t launch_hw(const Geometry &g, const SlabInputs &in, float *out, doubl
 }
 
 template <int SET>
-cudaError_t plan_set(const Geometry &g, Plan *pl) {
+double plan_set(const Geometry &g, int sms, double voxel_ns, size_t limit, FusePlan *pl) {
   switch (g.hw) {
-    case 1: return plan_hw<SET, 1>(g, pl);
-    case 2: return plan_hw<SET, 2>(g, pl);
-    case 3: return plan_hw<SET, 3>(g, pl);
-    case 4: return plan_hw<SET, 4>(g, pl);
-    case 5: return plan_hw<SET, 5>(g, pl);
-    default: return cudaErrorInvalidValue;
+    case 1: return plan_hw<SET, 1>(g, sms, voxel_ns, limit, pl);
+    case 2: return plan_hw<SET, 2>(g, sms, voxel_ns, limit, pl);
+    case 3: return plan_hw<SET, 3>(g, sms, voxel_ns, limit, pl);
+    case 4: return plan_hw<SET, 4>(g, sms, voxel_ns, limit, pl);
+    default: return plan_hw<SET, 5>(g, sms, voxel_ns, limit, pl);
   }
 }
 
-cudaError_t plan_any(const Geometry &g, int set, Plan *pl) {
+double plan_internal(const Geometry &g, int set, int sms, double voxel_ns, size_t limit,
+                     FusePlan *pl) {
   switch (set) {
-    case 0: return plan_set<0>(g, pl);
-    case 1: return plan_set<1>(g, pl);
-    case 2: return plan_set<2>(g, pl);
-    case 3: return plan_set<3>(g, pl);
-    case 4: return plan_set<4>(g, pl);
-    default: return cudaErrorInvalidValue;
+    case 1: return plan_set<1>(g, sms, voxel_ns, limit, pl);
+    case 2: return plan_set<2>(g, sms, voxel_ns, limit, pl);
+    case 3: return plan_set<3>(g, sms, voxel_ns, limit, pl);
+    case 4: return plan_set<4>(g, sms, voxel_ns, limit, pl);
+    case 5: return plan_set<5>(g, sms, voxel_ns, limit, pl);
+    case 6: return plan_set<6>(g, sms, voxel_ns, limit, pl);
+    case 7: return plan_set<7>(g, sms, voxel_ns, limit, pl);
+    default: return plan_set<0>(g, sms, voxel_ns, limit, pl);
   }
 }
 
 template <int SET>
 cudaError_t launch_set(const Geometry &g, const SlabInputs &in, float *out, double div,
-                       float *partial, int *err, const LaunchHooks &wt, int ib, int ie,
-                       cudaStream_t stream) {
+                       float *partial, int *err, const LaunchHooks &wt, const FusePlan &pl, int ib,
+                       int ie, cudaStream_t stream) {
   switch (g.hw) {
-    case 1: return launch_hw<SET, 1>(g, in, out, div, partial, err, wt, ib, ie, stream);
-    case 2: return launch_hw<SET, 2>(g, in, out, div, partial, err, wt, ib, ie, stream);
-    case 3: return launch_hw<SET, 3>(g, in, out, div, partial, err, wt, ib, ie, stream);
-    case 4: return launch_hw<SET, 4>(g, in, out, div, partial, err, wt, ib, ie, stream);
-    case 5: return launch_hw<SET, 5>(g, in, out, div, partial, err, wt, ib, ie, stream);
+    case 1: return launch_hw<SET, 1>(g, in, out, div, partial, err, wt, pl, ib, ie, stream);
+    case 2: return launch_hw<SET, 2>(g, in, out, div, partial, err, wt, pl, ib, ie, stream);
+    case 3: return launch_hw<SET, 3>(g, in, out, div, partial, err, wt, pl, ib, ie, stream);
+    case 4: return launch_hw<SET, 4>(g, in, out, div, partial, err, wt, pl, ib, ie, stream);
+    case 5: return launch_hw<SET, 5>(g, in, out, div, partial, err, wt, pl, ib, ie, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_any(const Geometry &g, const SlabInputs &in, float *out, double div,
+                       float *partial, int *err, const LaunchHooks &wt, const FusePlan &pl, int ib,
+                       int ie, cudaStream_t s) {
+  switch (pl.set) {
+    case 0: return launch_set<0>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 1: return launch_set<1>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 2: return launch_set<2>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 3: return launch_set<3>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 4: return launch_set<4>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 5: return launch_set<5>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 6: return launch_set<6>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
+    case 7: return launch_set<7>(g, in, out, div, partial, err, wt, pl, ib, ie, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 // Tiles and slab box sizes of one subject in the batched kernel.
 template <int SET, int HW>
-void batch_plan_hw(const Geometry &g, Plan *pl, int *yb, int *za, int *zl) {
+void batch_plan_hw(const Geometry &g, FusePlan *pl, int *yb, int *za, int *zl) {
   using T = BatchTileOf<SET, HW>;
   using C = Cfg<HW, T::RX, T::TZ>;
   tile_counts<T, HW>(g, pl);
@@ -946,8 +1027,9 @@ void batch_plan_hw(const Geometry &g, Plan *pl, int *yb, int *za, int *zl) {
 }
 
 template <int SET>
-cudaError_t batch_plan(int hw, const Geometry &g, Plan *pl, int *yb, int *za, int *zl) {
-  *pl = Plan{};
+cudaError_t batch_plan(int hw, const Geometry &g, FusePlan *pl, int *yb, int *za, int *zl) {
+  *pl = FusePlan{};
+  pl->groups = pl->atlas_groups = pl->splits = 1;  // many subjects fill the grid; no partial sums
   switch (hw) {
     case 5: batch_plan_hw<SET, 5>(g, pl, yb, za, zl); return cudaSuccess;
     case 4: batch_plan_hw<SET, 4>(g, pl, yb, za, zl); return cudaSuccess;
@@ -971,10 +1053,9 @@ cudaError_t launch_batch_set(const BatchSubjectIn *subs, int n, void *dev_scratc
   cudaError_t e;
   for (int k = 0; k < n; ++k) {
     const BatchSubjectIn &b = subs[order[k]];
-    Plan pl;
+    FusePlan pl;
     int yb, za, zl;
     if ((e = batch_plan<SET>(b.geom.hw, b.geom, &pl, &yb, &za, &zl)) != cudaSuccess) return e;
-    pl.groups = 1;  // many subjects fill the grid; no partial sums
     if ((e = make_slab_map(&maps[2 * k], b.in.atlas, b.geom.nx, b.geom.ny, b.geom.nz, b.geom.num,
                            b.in.pitch, yb, za)) != cudaSuccess)
       return e;
@@ -983,7 +1064,7 @@ cudaError_t launch_batch_set(const BatchSubjectIn *subs, int n, void *dev_scratc
       return e;
     SubjectView sv = subject_view(b.geom, b.in, b.out, b.div, nullptr, pl);
     sv.item_begin = total;
-    total += (b.geom.ix > 0 && b.geom.iy > 0 && b.geom.iz > 0) ? pl.ntiles : 0;
+    total += (b.geom.ix > 0 && b.geom.iy > 0 && b.geom.iz > 0) ? pl.tiles : 0;
     views[k] = sv;
   }
   // Device copies: maps first (64-byte aligned), then the subject views pointing at them.
@@ -1148,12 +1229,13 @@ cudaError_t launch_fuse_masked(const Geometry &g, const SlabInputs &in, double d
   if ((e = cudaMemsetAsync(count, 0, sizeof(int), stream)) != cudaSuccess) return e;
   masked_items_kernel<<<(ntiles + 255) / 256, 256, 0, stream>>>(masks, ntiles, items, count);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  Plan pl{};
+  FusePlan pl{};
   pl.tiles_y = ts.tiles_y;
   pl.tiles_x = ts.tiles_x;
   pl.tiles_z = ts.tiles_z;
-  pl.ntiles = ntiles;
+  pl.tiles = ntiles;
   pl.groups = 2;  // partial slots (the pair of each item), not a plan's atlas groups
+  pl.atlas_groups = pl.splits = 1;
   TmaParams p{};
   p.sv = subject_view(g, in, nullptr, div, partial, pl);
   p.sv.atlas_base = atlas_base;
@@ -1168,32 +1250,28 @@ cudaError_t launch_fuse_masked(const Geometry &g, const SlabInputs &in, double d
   return cudaGetLastError();
 }
 
-size_t fuse_tma_partial_bytes(const Geometry &g, int set) {
-  if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return 0;
-  Plan pl;
-  if (plan_any(g, set, &pl) != cudaSuccess || pl.groups <= 1) return 0;
-  return (size_t)pl.groups * 2 * (size_t)g.nvox() * sizeof(float);
-}
-
-cudaError_t fuse_tma_plan(const Geometry &g, int set, FusePlanInfo *info) {
-  *info = FusePlanInfo{0, 0, 0, 0, 0, 0, 0, 0};
+cudaError_t fuse_tma_plan(const Geometry &g, int set, size_t partial_limit, FusePlan *plan) {
+  *plan = FusePlan{};
+  if (g.hw < 1 || g.hw > 5 || set < 0 || set >= kTileSets) return cudaErrorInvalidValue;
   if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaSuccess;
-  Plan pl;
-  cudaError_t e = plan_any(g, set, &pl);
-  if (e != cudaSuccess) return e;
-  info->groups = pl.groups;
-  info->tiles = pl.ntiles;
-  info->ctas = pl.blocks;
-  info->rx = pl.rx;
-  info->tz = pl.tz;
-  info->partial_bytes =
-      pl.groups > 1 ? (size_t)pl.groups * 2 * (size_t)g.nvox() * sizeof(float) : 0;
-  info->tiles_z = pl.tiles_z;
-  info->tiles_xy = pl.tiles_y * pl.tiles_x;
+  const int sms = sm_count();
+  if (set != 0) {
+    plan_internal(g, set, sms, kTileCost[g.hw - 1][0], partial_limit, plan);
+    return cudaSuccess;
+  }
+  double best = -1.0;
+  for (int k = 0; k < 4; ++k) {
+    FusePlan p{};
+    const double t =
+        plan_internal(g, kTileChoices[k], sms, kTileCost[g.hw - 1][k], partial_limit, &p);
+    if (best >= 0.0 && t >= best) continue;
+    best = t;
+    *plan = p;
+  }
   return cudaSuccess;
 }
 
-int fuse_tma_planes_read(const Geometry &g, const FusePlanInfo &info, int ztiles) {
+int fuse_tma_planes_read(const Geometry &g, const FusePlan &info, int ztiles) {
   // z-tile tz reads the atlas MRI slab [2 tz TZ, 2 tz TZ + 2 TZ + 2 + 2 HW) (its first output
   // plane minus the box and window reach), the CT slab and the input taps lie inside it
   const long long n = (long long)ztiles * 2 * info.tz + 2 + 2 * g.hw;
@@ -1201,43 +1279,26 @@ int fuse_tma_planes_read(const Geometry &g, const FusePlanInfo &info, int ztiles
 }
 
 cudaError_t launch_fuse_tma(const Geometry &g, const SlabInputs &in, float *out, double div,
-                            float *partial, int *err, const LaunchHooks &wt, int set,
+                            float *partial, int *err, const LaunchHooks &wt, const FusePlan &plan,
                             cudaStream_t stream) {
   if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaSuccess;
-  switch (set) {
-    case 0: return launch_set<0>(g, in, out, div, partial, err, wt, -1, -1, stream);
-    case 1: return launch_set<1>(g, in, out, div, partial, err, wt, -1, -1, stream);
-    case 2: return launch_set<2>(g, in, out, div, partial, err, wt, -1, -1, stream);
-    case 3: return launch_set<3>(g, in, out, div, partial, err, wt, -1, -1, stream);
-    case 4: return launch_set<4>(g, in, out, div, partial, err, wt, -1, -1, stream);
-    default: return cudaErrorInvalidValue;
-  }
+  return launch_any(g, in, out, div, partial, err, wt, plan, -1, -1, stream);
 }
 
 cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, double div,
-                                  float *partial, int *err, int set, int item_begin, int item_end,
-                                  cudaStream_t stream) {
+                                  float *partial, int *err, const FusePlan &plan, int item_begin,
+                                  int item_end, cudaStream_t stream) {
   if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaSuccess;
   if (item_begin < 0) return cudaErrorInvalidValue;
   const LaunchHooks wt{0, nullptr, nullptr};
-  switch (set) {
-    case 0: return launch_set<0>(g, in, nullptr, div, partial, err, wt, item_begin, item_end, stream);
-    case 1: return launch_set<1>(g, in, nullptr, div, partial, err, wt, item_begin, item_end, stream);
-    case 2: return launch_set<2>(g, in, nullptr, div, partial, err, wt, item_begin, item_end, stream);
-    case 3: return launch_set<3>(g, in, nullptr, div, partial, err, wt, item_begin, item_end, stream);
-    case 4: return launch_set<4>(g, in, nullptr, div, partial, err, wt, item_begin, item_end, stream);
-    default: return cudaErrorInvalidValue;
-  }
+  return launch_any(g, in, nullptr, div, partial, err, wt, plan, item_begin, item_end, stream);
 }
 
-cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, int set, float *out,
-                                    int z_begin, int z_end, cudaStream_t stream) {
+cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, const FusePlan &plan,
+                                    float *out, int z_begin, int z_end, cudaStream_t stream) {
   if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaSuccess;
-  Plan pl;
-  cudaError_t e = plan_any(g, set, &pl);
-  if (e != cudaSuccess) return e;
-  if (pl.groups < 2) return cudaErrorInvalidValue;
-  return launch_combine_groups(g, partial, pl.groups, out, z_begin, z_end, stream);
+  if (plan.groups < 2) return cudaErrorInvalidValue;
+  return launch_combine_groups(g, partial, plan.groups, out, z_begin, z_end, stream);
 }
 
 namespace {

@@ -33,9 +33,9 @@ struct SlabInputs {
 };
 
 // TMA-staged plain FP32 fusion. Writes interior voxels of out only. *err (device) is set to a
-// non-zero code if a bounded wait gave up; the caller zeroes it beforehand. When the planner
-// splits the atlases into groups (to fill the persistent grid), `partial` must point to
-// fuse_tma_partial_bytes(g) bytes of device scratch; otherwise it may be null.
+// non-zero code if a bounded wait gave up; the caller zeroes it beforehand. When the plan has
+// two or more groups, `partial` must point to its partial_bytes of device scratch; otherwise it
+// may be null.
 // Hooks of one fusion launch. Testing hook for the bounded waits: when timeout_ns != 0, the first
 // CTA withholds its first copies, so its wait runs out after timeout_ns and the launch reports a
 // timeout. Timing hook: non-null start / stop events are recorded on the stream right before and
@@ -47,28 +47,36 @@ struct LaunchHooks {
 
 // Tile-shape sets compiled into the library (chosen per handle, see pct_autotune).
 constexpr int kTileSets = 5;
-size_t fuse_tma_partial_bytes(const Geometry &g, int set);
-struct FusePlanInfo {
-  int groups, tiles, ctas, rx, tz;
-  size_t partial_bytes;
-  int tiles_z, tiles_xy;  // tiles are numbered z-major: tile t has z-tile t / tiles_xy
+// How the plain kernel runs one volume: the register tile, the work items (tile x group) and the
+// partial sums. Groups are atlas groups times ranges of the window's rows (x offsets); item =
+// group * tiles + tile, group = atlas group * splits + range.
+struct FusePlan {
+  int set;                   // register tile (public sets 1-4; set 0 chooses 0 or 5-7 by shape)
+  int rx, tz;                // its x rows per warp and z planes per half warp
+  int tiles_y, tiles_x, tiles_z;
+  int tiles;                 // numbered z-major: tile t has z-tile t / (tiles_x * tiles_y)
+  int atlas_groups, splits;  // splits > 1 only when every atlas is a group
+  int groups;                // atlas_groups * splits
+  int ctas;                  // persistent grid
+  size_t partial_bytes;      // 0 with one group
 };
-cudaError_t fuse_tma_plan(const Geometry &g, int set, FusePlanInfo *info);
+// Plans with at most partial_limit bytes of partial sums (one group needs none).
+cudaError_t fuse_tma_plan(const Geometry &g, int set, size_t partial_limit, FusePlan *plan);
 cudaError_t launch_fuse_tma(const Geometry &g, const SlabInputs &in, float *out, double div,
-                            float *partial, int *err, const LaunchHooks &wt, int set,
+                            float *partial, int *err, const LaunchHooks &wt, const FusePlan &plan,
                             cudaStream_t stream);
-// Pipelined form of the same (plans with 2 or more atlas groups only): the work items
-// [item_begin, item_end) into the partial sums (item = group * tiles + tile);
-// launch_fuse_tma_combine adds the groups into out once every item has run. Lets the host start
-// on the first planes of the first group while the rest is uploaded.
+// Pipelined form of the same (plans with 2 or more groups only): the work items
+// [item_begin, item_end) into the partial sums; launch_fuse_tma_combine adds the groups into out
+// once every item has run. Lets the host start on the first planes of the first group while the
+// rest is uploaded.
 cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, double div,
-                                  float *partial, int *err, int set, int item_begin, int item_end,
-                                  cudaStream_t stream);
+                                  float *partial, int *err, const FusePlan &plan, int item_begin,
+                                  int item_end, cudaStream_t stream);
 // Planes [0, n) of the input and atlas volumes that the items of z-tiles [0, ztiles) read.
-int fuse_tma_planes_read(const Geometry &g, const FusePlanInfo &info, int ztiles);
+int fuse_tma_planes_read(const Geometry &g, const FusePlan &plan, int ztiles);
 // The combine of the output planes [z_begin, z_end) (clipped to the interior).
-cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, int set, float *out,
-                                    int z_begin, int z_end, cudaStream_t stream);
+cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, const FusePlan &plan,
+                                    float *out, int z_begin, int z_end, cudaStream_t stream);
 
 // Tiles of the plain kernel as the learned form's fallback sees them (NH = 11, tile set 0): tile
 // t = (tz * tiles_x + tx) * tiles_y + ty covers interior y [30 ty, 30 ty + 30), x rows
