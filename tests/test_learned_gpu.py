@@ -142,3 +142,23 @@ def test_training_reduces_the_loss(data):
     m.close()
     ts.close()
     assert l1 < 0.9 * l0, (l0, l1)
+
+
+@pytest.mark.parametrize("begin,count", [(0, 1), (3, 2), (1, 4), (0, 148), (5, 149), (2, 446)])
+def test_gradients_at_every_fill_of_a_pass(data, begin, count):
+    """Sample counts that leave a CTA's pass part-empty, give some CTAs one sample more than others,
+    or one sample each; float64 bound from the FP32 sums of the layer-wise check above."""
+    subs, keep, host = data
+    samples = random_samples(host, 450, 4)
+    ts = TrainSet(subs, samples)
+    t, _ = ts.targets()
+    m = Model(9)
+    loss, g = m.grads(ts, begin, count)
+    w = m.params(inference=True)
+    m.close()
+    ts.close()
+    pick = slice(begin, begin + count)
+    x = learned_ref.patches([h.img for h in host], [h.atlas_mri for h in host], samples[pick], None)
+    ref_loss, ref_g = learned_ref.loss_and_grads(w, x, t[pick])
+    assert loss == pytest.approx(ref_loss, rel=1e-4)
+    assert np.linalg.norm(g - ref_g) / np.linalg.norm(ref_g) < 1e-4
