@@ -101,7 +101,7 @@ __global__ void targets_kernel(const SubjectRef *__restrict__ subs, const int *_
 //    multiply-adds per row); nine warps take conv2 while the other three take conv3.
 // The gradient of conv1's output overwrites that output, and conv3's likewise, once the weight
 // gradients that read it are done. 4,096 samples: 13.8 ms with one output per thread and the
-// gradients in shared memory, 1.61 ms now (gradients read back, whole call).
+// gradients in shared memory, 1.33 ms now (gradients read back, whole call).
 
 constexpr int kTS = 3;  // samples per CTA pass: what fits beside the weights in 227 KB
 
@@ -119,7 +119,7 @@ constexpr int kSmall = kSmallHB + kHeads;  // biases, heads, head biases
 
 struct TrainSmem {
   float w1[27][kCin][kC];
-  float w[3][27][kC][kC];  // conv2..conv4
+  float w[3][27][kC][kC];  // conv2..conv4 (conv2 and conv3 with wgroup)
   __align__(16) float small[kSmall];   // biases [4][16], heads [33][16], head biases [33]
   __align__(16) float gsmall[kSmall];  // this CTA's gradient sums of the same
   __align__(16) SampleSmem s[kTS];
@@ -146,6 +146,12 @@ __device__ __forceinline__ float dot(const float4 &a, const float4 &b, float acc
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 
+// Place of the four-channel group cog of row ci of conv2's and conv3's weights: rotated within the
+// row by the row's own group, so that the four lanes that read four groups of one row (forward) and
+// the four that read one group of four rows (input gradients) both hit different banks. (Without:
+// half of all shared wavefronts were conflicts, 1.62 ms for the 4,096 samples.)
+__device__ __forceinline__ int wgroup(int ci, int cog) { return 4 * (cog ^ (ci >> 2)); }
+
 // One output row (SO positions along y, row (z, x)) and channels [4 cg, 4 cg + 4) of a 16 -> 16
 // convolution, over the input channel groups [g0, g1).
 template <int SI, int SO>
@@ -163,7 +169,7 @@ __device__ __forceinline__ void conv_row(const float (&w)[27][kC][kC], const flo
       for (int ky = 0; ky < 3; ++ky)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const float4 wv = ld4(&w[kzx * 3 + ky][4 * g + c][4 * cg]);
+          const float4 wv = ld4(&w[kzx * 3 + ky][4 * g + c][wgroup(4 * g, cg)]);
 #pragma unroll
           for (int y = 0; y < SO; ++y) axpy(acc[y], get(v[y + ky], c), wv);
         }
@@ -194,7 +200,7 @@ __device__ __forceinline__ void grad_row(const float (&w)[27][kC][kC], const flo
         for (int ky = 0; ky < 3; ++ky)
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4 wv = ld4(&w[(kz * 3 + kx) * 3 + ky][4 * cg + c][4 * g]);
+            const float4 wv = ld4(&w[(kz * 3 + kx) * 3 + ky][4 * cg + c][wgroup(4 * cg, g)]);
 #pragma unroll
             for (int y = 0; y < SO; ++y) acc[y + ky][c] = dot(wv, v[y], acc[y + ky][c]);
           }
@@ -254,7 +260,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     const int off = l == 0 ? kW2 : l == 1 ? kW3 : kW4;
     for (int i = tid; i < 27 * kC * kC; i += kTrainThreads) {
       const int k = i / (kC * kC), ci = (i / kC) % kC, co = i % kC;
-      S.w[l][k][ci][co] = __bfloat162float(wbf[off + (co * kC + ci) * 27 + k]);
+      S.w[l][k][ci][l < 2 ? wgroup(ci, co >> 2) + (co & 3) : co] =
+          __bfloat162float(wbf[off + (co * kC + ci) * 27 + k]);
     }
   }
   auto small_param = [](int i) {  // flat parameter index of a small one
