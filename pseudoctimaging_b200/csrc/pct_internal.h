@@ -138,7 +138,7 @@ cudaError_t launch(void *fn, unsigned grid, unsigned block, cudaStream_t stream,
 // runtime's entry-point query; NULL if the driver does not provide it.
 void *tensor_map_encoder();
 
-// NaN median fill (synchronous on `stream`: it reads back a counter after each round).
+// NaN median fill (synchronous on `stream`: it reads back its counters after each launch).
 // scratch must hold regularize_scratch_bytes(nx*ny*nz) bytes.
 size_t regularize_scratch_bytes(long long nvox);
 cudaError_t launch_regularize(float *vol, int nx, int ny, int nz, int nh, void *scratch,

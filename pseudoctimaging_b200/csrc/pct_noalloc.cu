@@ -4,7 +4,7 @@
 // for example applications that hand all device memory to their own pool allocator up front and
 // forbid other libraries from calling cudaMalloc (to avoid fragmentation and surprise
 // out-of-memory failures), or latency-critical pipelines that must not allocate after start-up.
-// The regular entry point takes its scratch (two index lists over the volume) from a handle,
+// The regular entry point takes its scratch (an index list over the volume) from a handle,
 // which allocates on first use; this one uses a fixed array that lives in the library instead.
 //
 // The array below is allocated when the CUDA runtime loads this library's device code on a GPU,
@@ -27,7 +27,7 @@
 namespace {
 
 // Largest volume this entry point accepts, and the scratch it needs: a 64-byte header of
-// counters plus two index lists of kMaxVoxels ints each (64 MiB in total).
+// counters plus kMaxVoxels index entries, twice over (64 MiB in total, as documented to callers).
 constexpr long long kMaxVoxels = 1LL << 23;
 constexpr size_t kScratchBytes = 64 + 2 * (size_t)kMaxVoxels * sizeof(int);
 

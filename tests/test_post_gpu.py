@@ -91,3 +91,51 @@ def test_pipeline_against_oracle_pipeline(handle, name):
     d = np.abs(got - ref)
     assert d.max() <= 17.0
     assert (d > 0).mean() < 0.01
+
+
+def _sweep(vol, nh):
+    """RegularizationStep in its sequential order on a copy (float64 median of float32 values)."""
+    v = vol.copy()
+    nz, nx, ny = v.shape
+    lo = (nh - 1) // 2 + 1
+    fills = 0
+    for z, x, y in np.argwhere(np.isnan(v)):
+        if lo <= z < nz - lo and lo <= x < nx - lo and lo <= y < ny - lo:
+            n = v[z - 1:z + 2, x - 1:x + 2, y - 1:y + 2]
+            n = n[~np.isnan(n)].astype(np.float64)
+            v[z, x, y] = np.float32(np.median(n))
+            fills += 1
+    return v, fills
+
+
+@pytest.mark.parametrize("shape,nh,holes", [((9, 9, 9), 7, 1), ((20, 33, 131), 3, 40),
+                                            ((30, 40, 150), 11, 60), ((24, 70, 138), 5, 4000)])
+def test_fill_follows_long_chains_in_sweep_order(handle, shape, nh, holes):
+    """Boxes of NaN of up to 12 voxels a side (chains of dependent fills), rows that end before and
+    after 128 columns, and lists longer than one voxel per warp: bit-exact."""
+    r = np.random.default_rng(holes)
+    nz, nx, ny = shape
+    lo = (nh - 1) // 2 + 1
+    vol = r.normal(50, 20, shape).astype(np.float32)
+    for _ in range(holes):
+        p = [int(r.integers(lo, n - lo)) for n in shape]
+        e = [int(r.integers(1, 13)) if holes < 100 else int(r.integers(1, 5)) for _ in shape]
+        vol[p[0]:p[0] + e[0], p[1]:p[1] + e[1], p[2]:p[2] + e[2]] = np.nan
+    clean = np.nan_to_num(vol, nan=7.0)
+    clean[lo:nz - lo, lo:nx - lo, lo:ny - lo] = vol[lo:nz - lo, lo:nx - lo, lo:ny - lo]
+    ref, fills = _sweep(clean, nh)
+    d = torch.from_numpy(clean).cuda()
+    got_fills = handle.regularize_device(d.data_ptr(), nx, ny, nz, nh)
+    assert np.array_equal(bits(d.cpu().numpy()), bits(ref))
+    assert got_fills == fills
+
+
+def test_fill_leaves_what_nothing_can_fill(handle):
+    """NaN in the border may leave voxels without any value around them: the call ends and every
+    voxel that a value reaches is filled."""
+    vol = torch.full((11, 11, 11), float("nan"), device="cuda")
+    assert handle.regularize_device(vol.data_ptr(), 11, 11, 11, 7) == 0
+    assert bool(vol.isnan().all())
+    vol[4, 4, 3] = 5.0  # a border value beside the first interior voxel
+    assert handle.regularize_device(vol.data_ptr(), 11, 11, 11, 7) == 27
+    assert bool((vol[4:7, 4:7, 4:7] == 5.0).all())
