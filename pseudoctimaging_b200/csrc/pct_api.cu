@@ -148,27 +148,36 @@ int select_device(pct_handle *h) {
 
 constexpr size_t kMaxTimedLaunches = 4096;  // pct_set_kernel_timing: pairs kept between reads
 
+// Whether `s` is being captured (no allocation may happen then).
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();  // (a legacy default stream while another one is captured)
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 // Plans the plain kernel and makes room for its partial sums. The plan keeps to what the handle's
 // memory cap leaves for them once its other buffers have grown by `others_grow` bytes, and to what
 // is there already when the stream is being captured (no allocation then) or the device has no
 // more: one group needs none, so a plan always exists.
 int plan_fusion(pct_handle *h, const pct::Geometry &g, size_t others_grow, cudaStream_t s,
-                pct::FusePlan *plan) {
+                pct::FusePlan *plan, const pct::OffsetRuns *runs = nullptr) {
+  auto make = [&](size_t limit) {
+    return runs ? pct::fuse_runs_plan(g, *runs, limit, plan)
+                : pct::fuse_tma_plan(g, h->tile_set, limit, plan);
+  };
   size_t limit = SIZE_MAX;
   if (h->mem_limit) {
     const size_t others = h->allocated - h->partial.bytes + others_grow;
     limit = h->mem_limit > others ? h->mem_limit - others : 0;
   }
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
-    cudaGetLastError();  // (a legacy default stream while another one is captured)
-    capturing = cudaStreamCaptureStatusActive;
-  }
-  if (capturing != cudaStreamCaptureStatusNone) limit = std::min(limit, h->partial.bytes);
-  PCT_CUDA(h, pct::fuse_tma_plan(g, h->tile_set, limit, plan));
+  if (is_capturing(s)) limit = std::min(limit, h->partial.bytes);
+  PCT_CUDA(h, make(limit));
   if (!plan->partial_bytes || !ensure(h, h->partial, plan->partial_bytes)) return PCT_OK;
   h->last_error.clear();
-  PCT_CUDA(h, pct::fuse_tma_plan(g, h->tile_set, h->partial.bytes, plan));
+  PCT_CUDA(h, make(h->partial.bytes));
   return PCT_OK;
 }
 
@@ -209,6 +218,55 @@ int learned_ran(pct_handle *h, const pct::Geometry &g, cudaStream_t s) {
   return PCT_OK;
 }
 
+// The centre prior on the plain kernel's tiles: its offsets are runs of dw around the centre, so the
+// kernel's planes and x boxes are shared between them, which the rescoring's items per row cannot
+// (192x208x96, 8 atlases, k = 81: 1.32 ms against 2.56). *done stays false where it does not apply and
+// the rescoring runs instead: k = 1, and stacks that would have to be repacked for TMA when the
+// memory cap, a capture or the device leaves no room for that.
+int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in, float *d_out,
+                       double div, cudaStream_t s, bool *done) {
+  *done = false;
+  pct::OffsetRuns runs;
+  const int k = h->learned_prior_k;
+  if (g.iy <= 0 || g.iz <= 0 || (long long)g.nz * g.nx * in.pitch >= (1LL << 31) - 1 ||
+      !pct::make_offset_runs(pct::learned::prior_offsets(k, g.hw), &runs))
+    return PCT_OK;
+  int st = ensure(h, h->err, 16);
+  if (st) return st;
+  const bool aligned = (in.pitch % 4 == 0) && (reinterpret_cast<uintptr_t>(in.atlas) % 16 == 0) &&
+                       (reinterpret_cast<uintptr_t>(in.label) % 16 == 0);
+  if (!aligned) {
+    const int pitch = pct::slab_pitch(g.ny);
+    const long long rows = (long long)g.num * g.nz * g.nx;
+    const size_t bytes = (size_t)rows * pitch * sizeof(float);
+    const bool there = h->atlas.bytes >= bytes && h->label.bytes >= bytes;
+    if (in.pitch != g.ny || (!there && is_capturing(s))) return PCT_OK;
+    if (ensure(h, h->atlas, bytes) || ensure(h, h->label, bytes)) {
+      h->last_error.clear();
+      return PCT_OK;
+    }
+    PCT_CUDA(h, pct::launch_pitch_copy(in.atlas, static_cast<float *>(h->atlas.ptr), rows, g.ny,
+                                       pitch, s));
+    PCT_CUDA(h, pct::launch_pitch_copy(in.label, static_cast<float *>(h->label.ptr), rows, g.ny,
+                                       pitch, s));
+    in = pct::SlabInputs{in.img, static_cast<const float *>(h->atlas.ptr),
+                         static_cast<const float *>(h->label.ptr), pitch};
+  }
+  pct::FusePlan plan;
+  if ((st = plan_fusion(h, g, 0, s, &plan, &runs))) return st;
+  int *err = static_cast<int *>(h->err.ptr);
+  PCT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), s));
+  // offsets evaluated per row of 30 voxels, as the rescoring counts them
+  const unsigned long long evaluated =
+      (unsigned long long)g.iz * g.ix * ((g.iy + 29) / 30) * k * g.num;
+  PCT_CUDA(h, pct::launch_fuse_runs(g, in, d_out, div, static_cast<float *>(h->partial.ptr), err,
+                                    plan, runs,
+                                    pct::learned::infer_counters(h->learned.ptr, g.nvox()),
+                                    evaluated, s));
+  *done = true;
+  return PCT_OK;
+}
+
 // The learned form: conv features, proposal and exact rescoring over all atlases (NH = 11).
 int launch_learned_path(pct_handle *h, const pct::Geometry &g, const pct::SlabInputs &in,
                         float *d_out, double div, cudaStream_t s) {
@@ -229,7 +287,10 @@ int launch_learned_path(pct_handle *h, const pct::Geometry &g, const pct::SlabIn
       return fail(h, PCT_ERR_UNSUPPORTED, "the centre prior needs at least 4 interior x-rows");
     int st = ensure(h, h->learned, pct::learned::infer_scratch_bytes(g));
     if (st) return st;
-    PCT_CUDA(h, pct::learned::launch_prior(g, in, d_out, div, h->learned_prior_k, h->learned.ptr, s));
+    bool done = false;
+    if ((st = launch_prior_tiles(h, g, in, d_out, div, s, &done))) return st;
+    if (!done)
+      PCT_CUDA(h, pct::learned::launch_prior(g, in, d_out, div, h->learned_prior_k, h->learned.ptr, s));
     return learned_ran(h, g, s);
   }
   if (pct::learned::model_device(h->model) != h->device)

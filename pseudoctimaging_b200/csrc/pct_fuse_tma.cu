@@ -32,7 +32,9 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "pct_internal.h"
@@ -60,7 +62,9 @@ __device__ __forceinline__ float fuse_result(float product, float sum_weight) {
 
 // ---------------------------------------------------------------- geometry of one variant
 
-template <int HW, int RX, int TZ>
+// LIST: an offset list of reach HW in a volume of any half window, so that a tile's slab may start at
+// any y modulo 4 (the plain kernel's start at 30 ty: 0 or 2).
+template <int HW, int RX, int TZ, bool LIST = false>
 struct Cfg {
   static constexpr int NQ = TZ + 2;          // D planes per half
   static constexpr int NR = RX + 2;          // D rows per warp
@@ -68,7 +72,7 @@ struct Cfg {
   static constexpr int XC = kWarps * RX;     // output rows per CTA
   // y extent of a slab row: lanes span 32 positions, +-HW for dv, +2 for the 16-byte
   // alignment of the TMA start coordinate (tile starts are 30*ty, i.e. 0 or 2 mod 4).
-  static constexpr int YB = (34 + 2 * HW + 3) / 4 * 4;
+  static constexpr int YB = ((LIST ? 35 : 34) + 2 * HW + 3) / 4 * 4;
   static constexpr int ZA = 2 * TZ + 2 + 2 * HW;  // atlas MRI planes per slab row
   static constexpr int ZL = 2 * TZ + 2 * HW;      // atlas CT planes per slab row
   static constexpr int RA = XC + 3;               // MRI ring: XC+2 rows in use + 1 prefetch
@@ -95,7 +99,7 @@ struct SubjectView {
   int tiles_y, tiles_x, ntiles;
   int groups, atlases_per_group;  // items = groups * ntiles (group-major)
   int splits;         // groups per atlas group: each takes a range of the window's x offsets
-  int hw;             // half window of this subject (batched kernel dispatch)
+  int hw, lo;         // half window of this subject (batched kernel dispatch), first interior index
   int item_begin;     // first global item of this subject (batched kernel)
   int atlas_base;     // first atlas of group 0 (a single-atlas launch over a tile list)
   float *acc_p, *acc_w;  // non-null: add each voxel's (product, sum_weight) into these instead
@@ -249,6 +253,71 @@ __device__ __forceinline__ void xbox_squares(const float2 (&d)[RX + 2], float2 (
   }
 }
 
+// One offset of the lane's voxels, y-pair layout: step jj of a ring period (compile-time), slab
+// plane offset so. Atlas plane t (= step + D plane) and label plane t (= step + output plane) live
+// in ring slot (jj + plane) % NQ.
+template <int HW, int RX, int TZ, bool AL, bool LR, bool LIST = false>
+__device__ __forceinline__ void step_yp(const float2 (&In)[TZ + 2][RX + 2], float2 (&P)[TZ][RX],
+                                        float2 (&W)[TZ][RX], float2 (&Aw)[TZ + 2][RX + 2],
+                                        float2 (&Lw)[TZ + 2][RX],
+                                        const uint32_t (&rowA)[RX + 2], const uint32_t (&rowL)[RX],
+                                        const uint32_t so, const int jj, const float2 scale2) {
+  using C = Cfg<HW, RX, TZ, LIST>;
+  constexpr int NQ = C::NQ, NR = C::NR;
+        {
+          const int sa = (jj + NQ - 1) % NQ;
+  #pragma unroll
+          for (int r = 0; r < NR; ++r)
+            Aw[sa][r] = lds_pair<AL>(rowA[r] + so + (NQ - 1) * C::PLANE);
+          if constexpr (LR) {
+            const int sl = (jj + TZ - 1) % NQ;
+  #pragma unroll
+            for (int r = 0; r < RX; ++r)
+              Lw[sl][r] = lds_pair<AL>(rowL[r] + so + (TZ - 1) * C::PLANE);
+          }
+        }
+        // Output planes two at a time: the x-box of D = (s A - s I)^2 for the planes they need
+        // (computed once, as late as possible, to keep few x-box sums live), then the z-box, the
+        // y-box (half-warp shuffles), the weight and the accumulators.
+        float2 g[NQ][RX];
+  #pragma unroll
+        for (int q = 0; q < TZ; q += 2) {
+  #pragma unroll
+          for (int pq = (q == 0 ? 0 : q + 2); pq < (q + 4 < NQ ? q + 4 : NQ); ++pq) {
+            const int sq = (pq + jj) % NQ;
+            float2 d[NR];
+  #pragma unroll
+            for (int r = 0; r < NR; ++r) d[r] = fma2(Aw[sq][r], scale2, In[pq][r]);  // s * (A - I)
+            xbox_squares<RX>(d, g[pq]);
+          }
+  #pragma unroll
+          for (int x = 0; x < RX; ++x) {
+            float2 S[2];
+            if (q + 1 < TZ) {
+              const float2 mid = add2(g[q + 1][x], g[q + 2][x]);
+              S[0] = add2(g[q][x], mid);
+              S[1] = add2(mid, g[q + 3][x]);
+            } else {
+              S[0] = add2(add2(g[q][x], g[q + 1][x]), g[q + 2][x]);
+            }
+  #pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              if (q + k >= TZ) break;
+              const float2 cc = S[k];
+              const float lft = __shfl_up_sync(0xffffffffu, cc.y, 1, 16);
+              const float rgt = __shfl_down_sync(0xffffffffu, cc.x, 1, 16);
+              const float m = cc.x + cc.y;
+              const float2 e = add2(make_float2(m, m), make_float2(lft, rgt));
+              const float2 w = make_float2(ex2_approx(-e.x), ex2_approx(-e.y));
+              const float2 lab = LR ? Lw[(q + k + jj) % NQ][x]
+                                    : lds_pair<AL>(rowL[x] + so + (q + k) * C::PLANE);
+              P[q + k][x] = fma2(w, lab, P[q + k][x]);
+              W[q + k][x] = add2(W[q + k][x], w);
+            }
+          }
+        }
+}
+
 // One dw sweep (all dw for fixed atlas, du, dv) of the lane's voxels, y-pair layout.
 // rowA[r] / rowL[r]: the lane's pair in plane 0 of its half's slab rows, at this dv.
 template <int HW, int RX, int TZ, bool AL, bool LR>
@@ -258,8 +327,7 @@ __device__ __forceinline__ void sweep_dw_yp(const float2 (&In)[TZ + 2][RX + 2],
                                             const uint32_t (&rowL)[RX], const float2 scale2) {
   using C = Cfg<HW, RX, TZ>;
   constexpr int NQ = C::NQ, NR = C::NR;
-  // Atlas plane t (= step + D plane) and label plane t (= step + output plane) live in slot
-  // (t + OFF) % NQ; at virtual step v = c*NQ + jj that is slot (jj + plane) % NQ.
+  // (plane t lives in slot (t + OFF) % NQ: virtual step v = c*NQ + jj, slot (jj + plane) % NQ)
   float2 Aw[NQ][NR];
   float2 Lw[NQ][RX];
 #pragma unroll
@@ -279,58 +347,33 @@ __device__ __forceinline__ void sweep_dw_yp(const float2 (&In)[TZ + 2][RX + 2],
     for (int jj = 0; jj < NQ; ++jj) {
       if (jj < C::OFF && c == 0) continue;
       const uint32_t so = (uint32_t)(c * NQ + jj - C::OFF) * C::PLANE;  // real step s = dw + HW
-      {
-        const int sa = (jj + NQ - 1) % NQ;
+      step_yp<HW, RX, TZ, AL, LR>(In, P, W, Aw, Lw, rowA, rowL, so, jj, scale2);
+    }
+  }
+}
+
+// The same sweep over the `len` planes from w0 on only (an offset list's run of dw for one du, dv).
+template <int HW, int RX, int TZ, bool AL>
+__device__ __forceinline__ void sweep_run_yp(const float2 (&In)[TZ + 2][RX + 2],
+                                             float2 (&P)[TZ][RX], float2 (&W)[TZ][RX],
+                                             const uint32_t (&rowA)[RX + 2],
+                                             const uint32_t (&rowL)[RX], const int len,
+                                             const float2 scale2) {
+  using C = Cfg<HW, RX, TZ, true>;
+  constexpr int NQ = C::NQ, NR = C::NR;
+  float2 Aw[NQ][NR];
+  float2 Lw[NQ][RX];
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-          Aw[sa][r] = lds_pair<AL>(rowA[r] + so + (NQ - 1) * C::PLANE);
-        if constexpr (LR) {
-          const int sl = (jj + TZ - 1) % NQ;
+  for (int t = 0; t < NQ - 1; ++t)
 #pragma unroll
-          for (int r = 0; r < RX; ++r)
-            Lw[sl][r] = lds_pair<AL>(rowL[r] + so + (TZ - 1) * C::PLANE);
-        }
-      }
-      // Output planes two at a time: the x-box of D = (s A - s I)^2 for the planes they need
-      // (computed once, as late as possible, to keep few x-box sums live), then the z-box, the
-      // y-box (half-warp shuffles), the weight and the accumulators.
-      float2 g[NQ][RX];
+    for (int r = 0; r < NR; ++r) Aw[t][r] = lds_pair<AL>(rowA[r] + t * C::PLANE);
+#pragma unroll 1
+  for (int c = 0; c < len; c += NQ) {
 #pragma unroll
-      for (int q = 0; q < TZ; q += 2) {
-#pragma unroll
-        for (int pq = (q == 0 ? 0 : q + 2); pq < (q + 4 < NQ ? q + 4 : NQ); ++pq) {
-          const int sq = (pq + jj) % NQ;
-          float2 d[NR];
-#pragma unroll
-          for (int r = 0; r < NR; ++r) d[r] = fma2(Aw[sq][r], scale2, In[pq][r]);  // s * (A - I)
-          xbox_squares<RX>(d, g[pq]);
-        }
-#pragma unroll
-        for (int x = 0; x < RX; ++x) {
-          float2 S[2];
-          if (q + 1 < TZ) {
-            const float2 mid = add2(g[q + 1][x], g[q + 2][x]);
-            S[0] = add2(g[q][x], mid);
-            S[1] = add2(mid, g[q + 3][x]);
-          } else {
-            S[0] = add2(add2(g[q][x], g[q + 1][x]), g[q + 2][x]);
-          }
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            if (q + k >= TZ) break;
-            const float2 cc = S[k];
-            const float lft = __shfl_up_sync(0xffffffffu, cc.y, 1, 16);
-            const float rgt = __shfl_down_sync(0xffffffffu, cc.x, 1, 16);
-            const float m = cc.x + cc.y;
-            const float2 e = add2(make_float2(m, m), make_float2(lft, rgt));
-            const float2 w = make_float2(ex2_approx(-e.x), ex2_approx(-e.y));
-            const float2 lab = LR ? Lw[(q + k + jj) % NQ][x]
-                                  : lds_pair<AL>(rowL[x] + so + (q + k) * C::PLANE);
-            P[q + k][x] = fma2(w, lab, P[q + k][x]);
-            W[q + k][x] = add2(W[q + k][x], w);
-          }
-        }
-      }
+    for (int jj = 0; jj < NQ; ++jj) {
+      if (jj > 0 && c + jj >= len) return;
+      const uint32_t so = (uint32_t)(c + jj) * C::PLANE;
+      step_yp<HW, RX, TZ, AL, false, true>(In, P, W, Aw, Lw, rowA, rowL, so, jj, scale2);
     }
   }
 }
@@ -346,10 +389,13 @@ struct Pipe {
 // Processes work item `item` (tile x atlas group) of subject `sv` with register tile (RX, TZ) in
 // layout LY (0: z-halves packed; 1: y-pairs, labels read per use; 2: y-pairs, labels in a
 // register ring). Returns false when a bounded wait gave up (the CTA must stop).
-template <int HW, int RX, int TZ, int LY, bool MASKED = false>
+// With `runs` (y-pairs, labels read per use) an item evaluates that offset list instead of the whole
+// window, and HW is the reach of the list rather than the volume's half window.
+template <int HW, int RX, int TZ, int LY, bool MASKED = false, bool LIST = false>
 __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &pp, int *err,
-                                         unsigned long long timeout_ns, int withhold_cta) {
-  using C = Cfg<HW, RX, TZ>;
+                                         unsigned long long timeout_ns, int withhold_cta,
+                                         const OffsetRuns *runs = nullptr) {
+  using C = Cfg<HW, RX, TZ, LIST>;
   constexpr int NQ = C::NQ, NR = C::NR, NS = C::NS;
   const uint32_t bar0 = pp.base, bar1 = pp.base + 8;
   const uint32_t ringA = pp.base + 128;
@@ -357,7 +403,7 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
   // (the shuffle tells the compiler that the warp index, and every ring address made from it, is
   // uniform over the warp)
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int lo = HW + 1;
+  const int lo = LIST ? sv.lo : HW + 1;
   const float2 scale2 = make_float2(sv.scale, sv.scale);
   int grp, t, a_first, natl;
   int j0 = 0, nj = NS;  // the item's x offsets du = j - HW, j in [j0, j0 + nj)
@@ -476,7 +522,24 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
 #pragma unroll
     for (int r = 0; r < RX; ++r)
       rowL[r] = ringL + (uint32_t)((warp * RX + r + j) % C::RL) * C::SLOT_L + lane_off;
-    if constexpr (LY == 0) {
+    if constexpr (LIST) {
+      static_assert(LY == 1, "offset lists run in the y-pair layout");
+#pragma unroll 1
+      for (int sv2 = 0; sv2 < NS; ++sv2) {
+        const int len = runs->len[j][sv2];
+        if (len == 0) continue;
+        const uint32_t at = (uint32_t)((sv2 - HW) * 4) + runs->w0[j][sv2] * C::PLANE;
+        uint32_t ra[NR], rl[RX];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) ra[r] = rowA[r] + at;
+#pragma unroll
+        for (int r = 0; r < RX; ++r) rl[r] = rowL[r] + at;
+        if ((sv2 + e) & 1)  // the pairs' 8-byte alignment also follows the slab's start
+          sweep_run_yp<HW, RX, TZ, false>(In, P, W, ra, rl, len, scale2);
+        else
+          sweep_run_yp<HW, RX, TZ, true>(In, P, W, ra, rl, len, scale2);
+      }
+    } else if constexpr (LY == 0) {
 #pragma unroll 1
       for (int dv = -HW; dv <= HW; ++dv) {
         uint32_t ra[NR], rl[RX];
@@ -582,6 +645,29 @@ __global__ void __launch_bounds__(kThreads, MB)
   p.sv.tmL = &tmL;
   for (int item = p.item_begin + blockIdx.x; item < p.item_end; item += gridDim.x) {
     if (!run_item<HW, RX, TZ, LY>(p.sv, item, pp, p.err, p.timeout_ns, p.withhold_cta)) {
+      pipe_drain(pp, p.timeout_ns);
+      return;
+    }
+  }
+}
+
+// An offset list (the centre prior) over the tiles of one subject. Counts its own evaluations
+// where pct_learned_stats reads them. Issue-bound like the full search, plus the first planes of each
+// run (a run of k = 81 has 3.9 offsets on average). y-pairs (2,6), 192x208x96, 8 atlases: k = 7
+// 0.25 ms (0.58 by the rescoring's items), k = 81 1.32 ms (2.56), k = 123 2.00 ms (3.78); (2,4) 0.30 /
+// 1.40 / 2.08, (3,4) 0.32 / 1.33 / 2.01.
+template <int HW, int RX, int TZ>
+__global__ void __launch_bounds__(kThreads, 1)
+    fuse_runs_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmL,
+                     TmaParams p, const __grid_constant__ OffsetRuns runs,
+                     unsigned long long *__restrict__ stats, unsigned long long evaluated) {
+  extern __shared__ unsigned char smem_raw[];
+  Pipe pp = pipe_init(smem_raw);
+  p.sv.tmA = &tmA;
+  p.sv.tmL = &tmL;
+  if (blockIdx.x == 0 && threadIdx.x < 2) stats[threadIdx.x] = threadIdx.x ? evaluated : 0;
+  for (int item = p.item_begin + blockIdx.x; item < p.item_end; item += gridDim.x) {
+    if (!run_item<HW, RX, TZ, 1, false, true>(p.sv, item, pp, p.err, p.timeout_ns, -1, &runs)) {
       pipe_drain(pp, p.timeout_ns);
       return;
     }
@@ -840,7 +926,7 @@ double expected_us(const Geometry &g, const FusePlan &pl, int slots, double voxe
 // Three groups or more are taken over fewer when they cost at most 3 % more: the host-pointer path
 // overlaps its uploads with the fusion group by group, and the FP32 sums are shorter.
 double choose_groups(const Geometry &g, int slots, double voxel_ns, size_t partial_limit,
-                     FusePlan *pl) {
+                     bool may_split, FusePlan *pl) {
   const int ns = g.nh;
   auto bytes_of = [&](int groups) {
     return groups > 1 ? (size_t)groups * 2 * (size_t)g.nvox() * sizeof(float) : 0;
@@ -861,7 +947,7 @@ double choose_groups(const Geometry &g, int slots, double voxel_ns, size_t parti
   };
   for (int a = 2; a <= g.num; ++a)
     if (g.num % a == 0) consider(a, 1);
-  for (int sp = 2; sp <= ns; ++sp) consider(g.num, sp);
+  for (int sp = 2; may_split && sp <= ns; ++sp) consider(g.num, sp);
   if (splits == 1 && agroups < 3)
     for (int a = 3; a <= g.num; ++a) {
       if (g.num % a) continue;
@@ -879,14 +965,15 @@ double choose_groups(const Geometry &g, int slots, double voxel_ns, size_t parti
 }
 
 template <int SET, int HW>
-double plan_hw(const Geometry &g, int sms, double voxel_ns, size_t partial_limit, FusePlan *pl) {
+double plan_hw(const Geometry &g, int sms, double voxel_ns, size_t partial_limit, FusePlan *pl,
+               bool may_split = true) {
   using T = TileOf<SET, HW>;
   // two CTAs share an SM's shared memory (228 KB, 1 KB reserved per CTA) and registers
   static_assert(T::MB > 1 || 2 * (Cfg<HW, T::RX, T::TZ>::SMEM + 1024) <= 228 * 1024, "2 CTAs per SM");
   tile_counts<T, HW>(g, pl);
   pl->set = SET;
   const int slots = sms * (T::MB > 1 ? T::MB : 2);
-  const double t = choose_groups(g, slots, voxel_ns, partial_limit, pl);
+  const double t = choose_groups(g, slots, voxel_ns, partial_limit, may_split, pl);
   const long long items = (long long)pl->tiles * pl->groups;
   pl->ctas = (int)(items < slots ? items : slots);
   return t;
@@ -911,6 +998,7 @@ SubjectView subject_view(const Geometry &g, const SlabInputs &in, float *out, do
   sv.splits = pl.splits;
   sv.atlases_per_group = g.num / pl.atlas_groups;
   sv.hw = g.hw;
+  sv.lo = g.lo;
   return sv;
 }
 
@@ -1140,6 +1228,99 @@ cudaError_t launch_prepared_batch(const BatchSetup &setup, cudaStream_t stream) 
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
+}
+
+bool make_offset_runs(const std::vector<std::array<int, 3>> &offsets, OffsetRuns *runs) {
+  int reach = 0;
+  for (const auto &o : offsets)
+    reach = std::max(reach, std::max(std::abs(o[0]), std::max(std::abs(o[1]), std::abs(o[2]))));
+  if (reach < 1 || reach > kMaxRunReach) return false;
+  *runs = OffsetRuns{};
+  runs->reach = reach;
+  runs->count = (int)offsets.size();
+  const int ns = 2 * reach + 1;
+  std::vector<char> has((size_t)ns * ns * ns, 0);
+  for (const auto &o : offsets) {
+    char &h = has[((size_t)(o[1] + reach) * ns + o[2] + reach) * ns + o[0] + reach];
+    if (h) return false;
+    h = 1;
+  }
+  for (int u = 0; u < ns; ++u)
+    for (int v = 0; v < ns; ++v) {
+      const char *h = &has[((size_t)u * ns + v) * ns];
+      int first = ns, last = -1, n = 0;
+      for (int w = 0; w < ns; ++w)
+        if (h[w]) {
+          first = std::min(first, w);
+          last = w;
+          ++n;
+        }
+      if (n && last - first + 1 != n) return false;  // not one run of dw
+      runs->w0[u][v] = (unsigned char)(n ? first : 0);
+      runs->len[u][v] = (unsigned char)n;
+    }
+  return true;
+}
+
+namespace {
+template <int SET, int HW>
+cudaError_t launch_runs_hw(const Geometry &g, const SlabInputs &in, float *out, double div,
+                           float *partial, int *err, const FusePlan &pl, const OffsetRuns &runs,
+                           unsigned long long *stats, unsigned long long evaluated,
+                           cudaStream_t stream) {
+  using T = TileOf<SET, HW>;
+  using C = Cfg<HW, T::RX, T::TZ, true>;
+  if (pl.groups > 1 && !partial) return cudaErrorInvalidValue;
+  auto kern = fuse_runs_kernel<HW, T::RX, T::TZ>;
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)) !=
+      cudaSuccess)
+    return e;
+  CUtensorMap tmA, tmL;
+  if ((e = make_slab_map(&tmA, in.atlas, g.nx, g.ny, g.nz, g.num, in.pitch, C::YB, C::ZA)) !=
+          cudaSuccess ||
+      (e = make_slab_map(&tmL, in.label, g.nx, g.ny, g.nz, g.num, in.pitch, C::YB, C::ZL)) !=
+          cudaSuccess)
+    return e;
+  TmaParams p{};
+  p.sv = subject_view(g, in, out, div, partial, pl);
+  p.err = err;
+  p.timeout_ns = 2000000000ull;
+  p.withhold_cta = -1;
+  p.item_end = pl.groups * pl.tiles;
+  kern<<<pl.ctas, kThreads, C::SMEM, stream>>>(tmA, tmL, p, runs, stats, evaluated);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return pl.groups > 1 ? launch_combine_groups(g, partial, pl.groups, out, stream) : cudaSuccess;
+}
+}  // namespace
+
+cudaError_t fuse_runs_plan(const Geometry &g, const OffsetRuns &runs, size_t partial_limit,
+                           FusePlan *plan) {
+  *plan = FusePlan{};
+  const int ns = 2 * runs.reach + 1;
+  if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaErrorInvalidValue;
+  // the tile's cost for a whole window of this reach, by the list's share of it; the runs are
+  // shorter, so that the first planes of each weigh more
+  const double cost = 1.2 * kTileCost[runs.reach - 1][2] * runs.count / ((double)ns * ns * ns);
+  const int sms = sm_count();
+  switch (runs.reach) {
+    case 1: plan_hw<6, 1>(g, sms, cost, partial_limit, plan, false); break;
+    case 2: plan_hw<6, 2>(g, sms, cost, partial_limit, plan, false); break;
+    default: plan_hw<6, 3>(g, sms, cost, partial_limit, plan, false); break;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_fuse_runs(const Geometry &g, const SlabInputs &in, float *out, double div,
+                             float *partial, int *err, const FusePlan &pl, const OffsetRuns &runs,
+                             unsigned long long *stats, unsigned long long evaluated,
+                             cudaStream_t s) {
+  switch (runs.reach) {
+    case 1: return launch_runs_hw<6, 1>(g, in, out, div, partial, err, pl, runs, stats, evaluated, s);
+    case 2: return launch_runs_hw<6, 2>(g, in, out, div, partial, err, pl, runs, stats, evaluated, s);
+    case 3: return launch_runs_hw<6, 3>(g, in, out, div, partial, err, pl, runs, stats, evaluated, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 TileShape fuse_tile_shape(const Geometry &g) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <array>
 #include <string>
 #include <vector>
 
@@ -77,6 +78,24 @@ int fuse_tma_planes_read(const Geometry &g, const FusePlan &plan, int ztiles);
 // The combine of the output planes [z_begin, z_end) (clipped to the interior).
 cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, const FusePlan &plan,
                                     float *out, int z_begin, int z_end, cudaStream_t stream);
+
+// A list of offsets as runs of dw: offsets (dw, du, dv) with du = j - reach, dv = i - reach and dw =
+// w0[j][i] - reach + n for n < len[j][i].
+constexpr int kMaxRunReach = 3;
+struct OffsetRuns {
+  int reach, count;
+  unsigned char w0[2 * kMaxRunReach + 1][8], len[2 * kMaxRunReach + 1][8];
+};
+// False when the list reaches further, holds only the centre, or is not one run per (du, dv).
+bool make_offset_runs(const std::vector<std::array<int, 3>> &offsets, OffsetRuns *runs);
+// The plain kernel over an offset list instead of the whole window (TMA-ready stacks): `stats` (two
+// device counters) receives {0, evaluated}. The plan never splits the window.
+cudaError_t fuse_runs_plan(const Geometry &g, const OffsetRuns &runs, size_t partial_limit,
+                           FusePlan *plan);
+cudaError_t launch_fuse_runs(const Geometry &g, const SlabInputs &in, float *out, double div,
+                             float *partial, int *err, const FusePlan &plan, const OffsetRuns &runs,
+                             unsigned long long *stats, unsigned long long evaluated,
+                             cudaStream_t stream);
 
 // Tiles of the plain kernel as the learned form's fallback sees them (NH = 11, tile set 0): tile
 // t = (tz * tiles_x + tx) * tiles_y + ty covers interior y [30 ty, 30 ty + 30), x rows
@@ -173,6 +192,9 @@ cudaError_t launch_learned(const Geometry &g, const void *weights, const SlabInp
                            double div, float conf_thr, int block, int level, bool every_voxel,
                            void *scratch, float *fb_partial, int *err,
                            const LearnedStreams *streams, cudaStream_t s);
+// The k offsets (dw, du, dv) of the NH^3 window (half width hw) nearest its centre, by squared
+// distance, ties in (dw, du, dv) order.
+std::vector<std::array<int, 3>> prior_offsets(int k, int hw);
 // The proposal baseline without a network (no convolutions, no proposal kernel): every voxel
 // rescores the k offsets of the window nearest its centre (1 <= k <= 125), with the same exact
 // FP32 rescoring as the learned form. Writes the interior of out.

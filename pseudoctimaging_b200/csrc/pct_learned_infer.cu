@@ -1961,8 +1961,6 @@ cudaError_t launch_learned(const Geometry &g, const void *weights, const SlabInp
   return cudaGetLastError();
 }
 
-// The k offsets (dw, du, dv) of the NH^3 window (half width hw) nearest its centre, by squared
-// distance, ties in (dw, du, dv) order.
 std::vector<std::array<int, 3>> prior_offsets(int k, int hw) {
   std::vector<std::array<int, 3>> all;
   for (int dw = -hw; dw <= hw; ++dw)
