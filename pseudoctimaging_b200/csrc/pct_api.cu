@@ -220,7 +220,7 @@ int learned_ran(pct_handle *h, const pct::Geometry &g, cudaStream_t s) {
 
 // The centre prior on the plain kernel's tiles: its offsets are runs of dw around the centre, so the
 // kernel's planes and x boxes are shared between them, which the rescoring's items per row cannot
-// (192x208x96, 8 atlases, k = 81: 1.32 ms against 2.56). *done stays false where it does not apply and
+// (192x208x96, 8 atlases, k = 81: 1.34 ms against 2.56). *done stays false where it does not apply and
 // the rescoring runs instead: k = 1, and stacks that would have to be repacked for TMA when the
 // memory cap, a capture or the device leaves no room for that.
 int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in, float *d_out,

@@ -83,6 +83,8 @@ struct Cfg {
   static constexpr uint32_t SLOT_L = (ROW_L + 127) / 128 * 128;
   static constexpr uint32_t PLANE = YB * 4;       // bytes between planes of a slab row
   static constexpr int SMEM = 128 + 128 + RA * SLOT_A + RL * SLOT_L;  // + alignment slack
+  // LIST: the threads' sums of whole atlases, behind the rings
+  static constexpr int SUMS = LIST ? kThreads * 4 * RX * TZ * (int)sizeof(float) : 0;
   static constexpr int NCH = (NS + NQ - 1) / NQ;  // ring periods per dw sweep
   static constexpr int OFF = NCH * NQ - NS;       // virtual steps skipped in the first period
 };
@@ -470,6 +472,31 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
       W[q][r] = make_float2(0.f, 0.f);
     }
 
+  // A list is short, so its sums are worth keeping short too: once 64 offsets or more are summed at
+  // the end of an atlas they are added to the thread's own sums in shared memory (one thread's
+  // column, no conflicts) and start again, as if each atlas had been summed by itself.
+  int summed = 0;
+  bool kept = false;
+  const uint32_t sums = ringL + C::RL * C::SLOT_L + (uint32_t)tid * 4u;
+  auto keep_sums = [&](bool restart) {
+#pragma unroll
+    for (int q = 0; q < TZ; ++q)
+#pragma unroll
+      for (int r = 0; r < RX; ++r)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          float2 &v = k ? W[q][r] : P[q][r];
+          float *at = static_cast<float *>(__cvta_shared_to_generic(
+              sums + (uint32_t)(((q * RX + r) * 2 + k) * 2 * kThreads * 4)));
+          if (kept) v = make_float2(at[0] + v.x, at[kThreads] + v.y);
+          if (restart) {
+            at[0] = v.x;
+            at[kThreads] = v.y;
+            v = make_float2(0.f, 0.f);
+          }
+        }
+  };
+
   int a = a_first;
   for (int i = 0; i < T; ++i, ++pp.gstep) {
     const int ai = i / nj, j = j0 + i - ai * nj;
@@ -539,6 +566,11 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
         else
           sweep_run_yp<HW, RX, TZ, true>(In, P, W, ra, rl, len, scale2);
       }
+      if (j == j0 + nj - 1 && i + 1 < T && (summed += runs->count) >= 64) {
+        keep_sums(true);
+        kept = true;
+        summed = 0;
+      }
     } else if constexpr (LY == 0) {
 #pragma unroll 1
       for (int dv = -HW; dv <= HW; ++dv) {
@@ -574,6 +606,9 @@ __device__ __forceinline__ bool run_item(const SubjectView &sv, int item, Pipe &
   }
   __syncthreads();  // a timeout in the item's last step is seen here
   if (*pp.abort_flag) return false;
+  if constexpr (LIST) {
+    if (kept) keep_sums(false);
+  }
 
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -654,8 +689,9 @@ __global__ void __launch_bounds__(kThreads, MB)
 // An offset list (the centre prior) over the tiles of one subject. Counts its own evaluations
 // where pct_learned_stats reads them. Issue-bound like the full search, plus the first planes of each
 // run (a run of k = 81 has 3.9 offsets on average). y-pairs (2,6), 192x208x96, 8 atlases: k = 7
-// 0.25 ms (0.58 by the rescoring's items), k = 81 1.32 ms (2.56), k = 123 2.00 ms (3.78); (2,4) 0.30 /
-// 1.40 / 2.08, (3,4) 0.32 / 1.33 / 2.01.
+// 0.25 ms (0.58 by the rescoring's items), k = 81 1.34 ms (2.56), k = 123 2.03 ms (3.78); (2,4) 0.30 /
+// 1.40 / 2.08, (3,4) 0.32 / 1.33 / 2.01 (without the sums kept per 64 offsets, which cost 1.5 % and
+// halve the error against FP64: 8.1e-8 instead of 1.5e-7).
 template <int HW, int RX, int TZ>
 __global__ void __launch_bounds__(kThreads, 1)
     fuse_runs_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmL,
@@ -1273,7 +1309,9 @@ cudaError_t launch_runs_hw(const Geometry &g, const SlabInputs &in, float *out, 
   if (pl.groups > 1 && !partial) return cudaErrorInvalidValue;
   auto kern = fuse_runs_kernel<HW, T::RX, T::TZ>;
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)) !=
+  constexpr int smem = C::SMEM + C::SUMS;
+  static_assert(2 * (smem + 1024) <= 228 * 1024, "2 CTAs per SM");
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=
       cudaSuccess)
     return e;
   CUtensorMap tmA, tmL;
@@ -1288,7 +1326,7 @@ cudaError_t launch_runs_hw(const Geometry &g, const SlabInputs &in, float *out, 
   p.timeout_ns = 2000000000ull;
   p.withhold_cta = -1;
   p.item_end = pl.groups * pl.tiles;
-  kern<<<pl.ctas, kThreads, C::SMEM, stream>>>(tmA, tmL, p, runs, stats, evaluated);
+  kern<<<pl.ctas, kThreads, smem, stream>>>(tmA, tmL, p, runs, stats, evaluated);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return pl.groups > 1 ? launch_combine_groups(g, partial, pl.groups, out, stream) : cudaSuccess;
 }
