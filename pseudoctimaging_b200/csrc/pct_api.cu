@@ -1238,7 +1238,7 @@ int pct_error_stats_device(pct_handle *h, const float *d_a, const float *d_b, in
 
 struct pct_batch {
   pct_handle *h = nullptr;
-  DevBuf stage, meta, err;
+  DevBuf stage, meta, err, partial;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   size_t bytes = 0;
@@ -1300,6 +1300,22 @@ int stage_batch(pct_handle *h, const pct_subject *subs, int n, const std::vector
   return PCT_OK;
 }
 
+// Plans a batch's atlas groups within what the handle's memory cap leaves for `buf` and makes room
+// for their partial sums; without it every subject is one group, which needs none.
+int plan_batch(pct_handle *h, const std::vector<pct::Geometry> &geo, int set, DevBuf &buf,
+               pct::BatchPlan *plan) {
+  size_t limit = SIZE_MAX;
+  if (h->mem_limit) {
+    const size_t others = h->allocated - buf.bytes;
+    limit = h->mem_limit > others ? h->mem_limit - others : 0;
+  }
+  PCT_CUDA(h, pct::plan_batch(geo.data(), (int)geo.size(), set, limit, plan));
+  if (!plan->partial_bytes || !ensure(h, buf, plan->partial_bytes)) return PCT_OK;
+  h->last_error.clear();
+  PCT_CUDA(h, pct::plan_batch(geo.data(), (int)geo.size(), set, 0, plan));
+  return PCT_OK;
+}
+
 int run_batch_once(pct_handle *h, const pct_subject *subs, int n, int set, cudaStream_t s) {
   std::vector<pct::Geometry> geo;
   int st = check_subjects(h, subs, n, geo);
@@ -1311,10 +1327,13 @@ int run_batch_once(pct_handle *h, const pct_subject *subs, int n, int set, cudaS
     return st;
   std::vector<pct::BatchSubjectIn> in;
   if ((st = stage_batch(h, subs, n, geo, h->batch_stage.ptr, in, s))) return st;
+  pct::BatchPlan plan;
+  if ((st = plan_batch(h, geo, set, h->partial, &plan))) return st;
   int *err = static_cast<int *>(h->err.ptr);
-  PCT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), s));
+  PCT_CUDA(h, cudaMemsetAsync(err, 0, 2 * sizeof(int), s));
   pct::BatchSetup setup;
-  PCT_CUDA(h, pct::prepare_batch(in.data(), n, set, h->batch_meta.ptr, err, s, &setup));
+  PCT_CUDA(h, pct::prepare_batch(in.data(), n, set, plan, static_cast<float *>(h->partial.ptr),
+                                 h->batch_meta.ptr, err, s, &setup));
   PCT_CUDA(h, pct::launch_prepared_batch(setup, s));
   return PCT_OK;
 }
@@ -1416,14 +1435,17 @@ int pct_batch_create(pct_handle *h, const pct_subject *subjects, int n, void *st
   if ((st = ensure(h, b->stage, batch_stage_bytes(subjects, n) + 256)) ||
       (st = ensure(h, b->meta, pct::batch_scratch_bytes(n))) || (st = ensure(h, b->err, 16)))
     return cleanup(st);
-  b->bytes = b->stage.bytes + b->meta.bytes + b->err.bytes;
+  pct::BatchPlan plan;
+  if ((st = plan_batch(h, geo, h->tile_set, b->partial, &plan))) return cleanup(st);
+  b->bytes = b->stage.bytes + b->meta.bytes + b->err.bytes + b->partial.bytes;
   std::vector<pct::BatchSubjectIn> in;
   pct::BatchSetup setup;
   // Subject table and tensor maps are uploaded once, before capture.
   {
     std::vector<pct::BatchSubjectIn> probe;
     if ((st = stage_batch(h, subjects, n, geo, b->stage.ptr, probe, s))) return cleanup(st);
-    cudaError_t e = pct::prepare_batch(probe.data(), n, h->tile_set, b->meta.ptr,
+    cudaError_t e = pct::prepare_batch(probe.data(), n, h->tile_set, plan,
+                                       static_cast<float *>(b->partial.ptr), b->meta.ptr,
                                        static_cast<int *>(b->err.ptr), s, &setup);
     if (e != cudaSuccess) return cleanup(cuda_fail(h, e, "prepare_batch"));
   }
@@ -1432,7 +1454,7 @@ int pct_batch_create(pct_handle *h, const pct_subject *subjects, int n, void *st
   if (e != cudaSuccess) return cleanup(cuda_fail(h, e, "cudaStreamBeginCapture"));
   st = stage_batch(h, subjects, n, geo, b->stage.ptr, in, s);
   if (!st) {
-    e = cudaMemsetAsync(b->err.ptr, 0, sizeof(int), s);
+    e = cudaMemsetAsync(b->err.ptr, 0, 2 * sizeof(int), s);
     if (e == cudaSuccess) e = pct::launch_prepared_batch(setup, s);
   }
   cudaGraph_t g = nullptr;
@@ -1474,7 +1496,7 @@ int pct_batch_destroy(pct_batch *b) {
   if (b->h) cudaSetDevice(b->h->device);
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  for (DevBuf *d : {&b->stage, &b->meta, &b->err})
+  for (DevBuf *d : {&b->stage, &b->meta, &b->err, &b->partial})
     if (d->ptr) {
       cudaFree(d->ptr);
       if (b->h) b->h->allocated -= d->bytes;

@@ -126,13 +126,22 @@ struct BatchSetup {
   int items = 0, blocks = 0, smem = 0, set = 0;
   void *bp_subjects = nullptr;
   int bp_nsub = 0;
-  int *bp_err = nullptr;
+  int *bp_err = nullptr;  // status word, then the counter of items taken (both zero at launch)
+  bool combine = false;   // some subject runs in atlas groups: their sums are combined afterwards
 };
+// Atlas groups per subject (in the caller's order) and the partial sums they need.
+struct BatchPlan {
+  std::vector<int> groups;
+  size_t partial_bytes = 0;
+};
+cudaError_t plan_batch(const Geometry *geoms, int n, int set, size_t partial_limit, BatchPlan *plan);
 size_t batch_scratch_bytes(int n);
 // Plans the batch and uploads its subject table and tensor maps to dev_scratch (synchronous).
-cudaError_t prepare_batch(const BatchSubjectIn *subs, int n, int set, void *dev_scratch, int *err,
-                          cudaStream_t stream, BatchSetup *setup);
-// Enqueues the persistent batch kernel (graph-capturable: no host work beyond the launch).
+cudaError_t prepare_batch(const BatchSubjectIn *subs, int n, int set, const BatchPlan &plan,
+                          float *partial, void *dev_scratch, int *err, cudaStream_t stream,
+                          BatchSetup *setup);
+// Enqueues the persistent batch kernel and the combine (graph-capturable: no host work beyond the
+// launches). The caller zeroes the two words at `err` before it.
 cudaError_t launch_prepared_batch(const BatchSetup &setup, cudaStream_t stream);
 
 // dst[r*pitch + c] = src[r*ny + c] for r < rows, c < ny.

@@ -114,3 +114,36 @@ def test_batch_rejects_windows_it_does_not_compile(handle):
     with pytest.raises(pct.PctError) as e:
         handle.synthesize_batch(subs)
     assert e.value.status == -4
+
+
+@pytest.mark.parametrize("specs", [
+    # long items beside short ones, prime atlas counts, one subject with an empty interior
+    [(40, 44, 36, 7, 11, 21), (30, 33, 28, 1, 7, 22), (12, 40, 30, 2, 11, 23), (36, 40, 31, 6, 9, 24)],
+    [(41, 46, 30, 5, 7, 25)]])
+def test_batch_in_atlas_groups_with_and_without_room(specs):
+    """Subjects split into atlas groups (partial sums, combined per subject) against the single-subject
+    path, and the same batch under a cap that leaves no room for the sums (one group each)."""
+    subs, host, dev = make_batch(specs)
+    with pct.Handle(0) as h:
+        h.synthesize_batch(subs)
+        h.device_status()
+        free = [out.clone() for _, out in dev]
+    with pct.Handle(0) as h:
+        lim = 1 << 12
+        while True:  # the smallest cap that runs leaves nothing for partial sums
+            h.set_memory_limit(lim)
+            try:
+                h.synthesize_batch(subs)
+                break
+            except pct.PctError as e:
+                assert e.status == -3
+                lim += lim // 16
+        h.device_status()
+        capped = [out.clone() for _, out in dev]
+        h.set_memory_limit(0)
+        for (nx, ny, nz, num, nh, _), (s, lab), a, b in zip(specs, host, free, capped):
+            single = h.synthesize(s.img, s.atlas_mri, lab, nh, 337.5)
+            for got in (a.cpu().numpy(), b.cpu().numpy()):
+                assert np.array_equal(np.isnan(got), np.isnan(single))
+                np.testing.assert_allclose(np.nan_to_num(got), np.nan_to_num(single), rtol=2e-5,
+                                           atol=1e-5)
