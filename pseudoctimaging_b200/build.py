@@ -34,7 +34,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", f"-ccbin={HOST_CXX}", "-Xcompiler", 
 LIB_SOURCES = ["pct_api.cu", "pct_fuse_tma.cu", "pct_pointwise.cu", "pct_regularize.cu",
                "pct_noalloc.cu", "pct_synth.cpp", "pct_io.cpp", "pct_learned_train.cu",
                "pct_learned_api.cu", "pct_learned_infer.cu", "pct_tc_fuse.cu", "pct_jit.cpp",
-               "pct_mat.cpp"]
+               "pct_mat.cpp", "pct_stage.cpp"]
 # Device sources that are also compiled at run time (NVRTC): each is embedded as a string in
 # _build/<stem>_src.inc, which the library sources include.
 EMBEDDED = ["pct_rescore.cuh"]

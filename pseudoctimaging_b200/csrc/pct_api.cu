@@ -12,6 +12,7 @@
 
 #include "pct_b200.h"
 #include "pct_internal.h"
+#include "pct_stage.h"
 
 namespace {
 
@@ -53,6 +54,7 @@ struct pct_handle {
   bool time_kernels = false;              // pct_set_kernel_timing
   std::vector<cudaEvent_t> kt_ev;         // start / stop pairs around timed fusion launches
   size_t kt_used = 0;                     // pairs recorded since the last pct_kernel_time
+  pct::HostStager stager;                 // pageable uploads and downloads of host-pointer calls
   std::string last_error;
 };
 
@@ -388,6 +390,32 @@ int read_device_status(pct_handle *h, cudaStream_t s) {
   return PCT_OK;
 }
 
+// Ends a call's staged uploads on every way out of it.
+struct StageScope {
+  pct::HostStager &stager;
+  ~StageScope() { stager.end(); }
+};
+
+// One upload of a host-pointer call, through the handle's staging when the call began it.
+cudaError_t upload(pct_handle *h, void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  if (h->stager.active()) return h->stager.copy(dst, src, bytes, s);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+}
+
+// One download: complete on return into pageable memory (as a direct copy there is), enqueued into
+// pinned memory.
+cudaError_t download(pct_handle *h, void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  if (h->stager.takes(dst, bytes)) return h->stager.download(h->device, dst, src, bytes, s);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+}
+
+// Begins staging the three uploads of the one-upload path.
+void begin_uploads(pct_handle *h, const pct::Geometry &g, const float *img, const float *atlas,
+                   const float *label) {
+  const size_t vol = (size_t)g.nvox() * sizeof(float);
+  h->stager.begin(h->device, {{img, vol}, {atlas, vol * g.num}, {label, vol * g.num}});
+}
+
 // Copies host atlas volumes [num*nz*nx][ny] into a pitched device stack for TMA: one
 // contiguous host->device copy (full PCIe/C2C rate) into a staging buffer, then an on-device
 // repack. When ny is already a multiple of 4 the copy lands in place.
@@ -399,11 +427,11 @@ int stage_pitched_h2d(pct_handle *h, DevBuf &buf, const float *src, const pct::G
   if (st) return st;
   const size_t bytes = rows * g.ny * sizeof(float);
   if (pitch == g.ny) {
-    PCT_CUDA(h, cudaMemcpyAsync(buf.ptr, src, bytes, cudaMemcpyHostToDevice, s));
+    PCT_CUDA(h, upload(h, buf.ptr, src, bytes, s));
     return PCT_OK;
   }
   if ((st = ensure(h, h->stage, bytes))) return st;
-  PCT_CUDA(h, cudaMemcpyAsync(h->stage.ptr, src, bytes, cudaMemcpyHostToDevice, s));
+  PCT_CUDA(h, upload(h, h->stage.ptr, src, bytes, s));
   PCT_CUDA(h, pct::launch_pitch_copy(static_cast<const float *>(h->stage.ptr),
                                      static_cast<float *>(buf.ptr), (long long)rows, g.ny, pitch, s));
   return PCT_OK;
@@ -425,10 +453,10 @@ int stage_pitched_slice(pct_handle *h, DevBuf &buf, float *stage_base, const flo
     const float *from = src + first_row * g.ny;
     const size_t bytes = rows * g.ny * sizeof(float);
     if (pitch == g.ny) {
-      PCT_CUDA(h, cudaMemcpyAsync(dst, from, bytes, cudaMemcpyHostToDevice, s));
+      PCT_CUDA(h, upload(h, dst, from, bytes, s));
     } else {
       float *stage = stage_base + first_row * g.ny;
-      PCT_CUDA(h, cudaMemcpyAsync(stage, from, bytes, cudaMemcpyHostToDevice, s));
+      PCT_CUDA(h, upload(h, stage, from, bytes, s));
       PCT_CUDA(h, pct::launch_pitch_copy(stage, dst, (long long)rows, g.ny, pitch, s));
     }
     if (normalize) PCT_CUDA(h, pct::launch_normalize_labels(dst, rows * pitch, s));
@@ -569,10 +597,8 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     const Part &p = parts[k];
     if (p.z1 > p.z0) {
       if (p.with_img)
-        PCT_CUDA(h, cudaMemcpyAsync(static_cast<float *>(h->img.ptr) + p.z0 * plane,
-                                    img + p.z0 * plane,
-                                    (size_t)(p.z1 - p.z0) * plane * sizeof(float),
-                                    cudaMemcpyHostToDevice, cs));
+        PCT_CUDA(h, upload(h, static_cast<float *>(h->img.ptr) + p.z0 * plane, img + p.z0 * plane,
+                           (size_t)(p.z1 - p.z0) * plane * sizeof(float), cs));
       int r = stage_pitched_slice(h, h->atlas, stage_mri, atlas, g, p.a0, p.a1, p.z0, p.z1, false,
                                   cs);
       if (!r)
@@ -596,13 +622,27 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     PCT_CUDA(h, cudaStreamWaitEvent(os, done(k), 0));
     PCT_CUDA(h, cudaStreamWaitEvent(os, done(k - 1), 0));
     PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, p.o0, p.o1, os));
-    PCT_CUDA(h, cudaMemcpyAsync(host_out + p.o0 * plane, d_out + p.o0 * plane,
-                                (size_t)(p.o1 - p.o0) * plane * sizeof(float),
-                                cudaMemcpyDeviceToHost, os));
+    PCT_CUDA(h, download(h, host_out + p.o0 * plane, d_out + p.o0 * plane,
+                         (size_t)(p.o1 - p.o0) * plane * sizeof(float), os));
     return PCT_OK;
   };
+  // The uploads in the order that run_part takes them (stage_pitched_slice: whole atlases are one
+  // run, a plane range one per atlas).
+  std::vector<pct::HostStager::Job> jobs;
+  for (const Part &p : parts) {
+    if (p.z1 <= p.z0) continue;
+    const size_t bytes = (size_t)(p.z1 - p.z0) * plane * sizeof(float);
+    if (p.with_img) jobs.push_back({img + p.z0 * plane, bytes});
+    const bool whole = p.z0 == 0 && p.z1 == g.nz;
+    for (const float *stack : {atlas, atlas_ct})
+      for (int a = p.a0; a < (whole ? p.a0 + 1 : p.a1); ++a)
+        jobs.push_back({stack + ((size_t)a * g.nz + p.z0) * plane, whole ? bytes * (p.a1 - p.a0) : bytes});
+  }
+  StageScope staging{h->stager};
+  h->stager.begin(h->device, jobs);
   st = PCT_OK;
   for (size_t k = 0; k < parts.size() && !st; ++k) st = run_part(k);
+  h->stager.end();
   for (size_t k = 1; k < parts.size() && !st; ++k)
     if (parts[k].o1 > parts[k].o0) st = run_output(k);
   // join (on failure too, so that nothing of this call is still running on the other streams
@@ -989,15 +1029,18 @@ int pct_synthesize(pct_handle *h, const float *img, const float *atlas, const fl
     if (st != PCT_ERR_UNSUPPORTED) return st;
     h->last_error.clear();
   }
-  PCT_CUDA(h, cudaMemcpyAsync(h->img.ptr, img, vol, cudaMemcpyHostToDevice, s));
+  StageScope staging{h->stager};
+  begin_uploads(h, g, img, atlas, atlas_label);
+  PCT_CUDA(h, upload(h, h->img.ptr, img, vol, s));
   if ((st = stage_pitched_h2d(h, h->atlas, atlas, g, s)) ||
       (st = stage_pitched_h2d(h, h->label, atlas_label, g, s)))
     return st;
+  h->stager.end();
   pct::SlabInputs in{static_cast<const float *>(h->img.ptr), static_cast<const float *>(h->atlas.ptr),
                      static_cast<const float *>(h->label.ptr), pct::slab_pitch(g.ny)};
   if ((st = launch_path(h, g, in, static_cast<float *>(h->out.ptr), div, exec_choice, s)))
     return st;
-  PCT_CUDA(h, cudaMemcpyAsync(label_segmentation, h->out.ptr, vol, cudaMemcpyDeviceToHost, s));
+  PCT_CUDA(h, download(h, label_segmentation, h->out.ptr, vol, s));
   PCT_CUDA(h, cudaStreamSynchronize(s));
   return read_device_status(h, s);
 }
@@ -1132,10 +1175,13 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
            : PCT_ERR_UNSUPPORTED;
   if (st == PCT_ERR_UNSUPPORTED) {  // one upload, then the path
     h->last_error.clear();
-    PCT_CUDA(h, cudaMemcpyAsync(d_img, img, vol, cudaMemcpyHostToDevice, s));
+    StageScope staging{h->stager};
+    begin_uploads(h, g, img, atlas_mri, atlas_ct_hu);
+    PCT_CUDA(h, upload(h, d_img, img, vol, s));
     if ((st = stage_pitched_h2d(h, h->atlas, atlas_mri, g, s)) ||
         (st = stage_pitched_h2d(h, h->label, atlas_ct_hu, g, s)))
       return st;
+    h->stager.end();
     const int pitch = pct::slab_pitch(g.ny);
     // Label normalisation over the whole pitched stack (padding columns are never read).
     PCT_CUDA(h, pct::launch_normalize_labels(static_cast<float *>(h->label.ptr),
@@ -1153,7 +1199,7 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
     PCT_CUDA(h, pct::launch_regularize(d_out, nx, ny, nz, nh, h->scratch.ptr, s, &f, &rounds));
     PCT_CUDA(h, pct::launch_finalize_hu(d_out, (size_t)g.nvox(), s));
   }
-  PCT_CUDA(h, cudaMemcpyAsync(out, d_out, vol, cudaMemcpyDeviceToHost, s));
+  PCT_CUDA(h, download(h, out, d_out, vol, s));
   PCT_CUDA(h, cudaStreamSynchronize(s));
   return PCT_OK;
 }

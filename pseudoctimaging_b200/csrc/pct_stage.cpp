@@ -1,0 +1,269 @@
+// See pct_stage.h. Hand-over: chunk i uses slot i % kSlots. Upload: a worker waits until chunk
+// i - kSlots has been issued and its transfer (the slot's event) is done, fills the slot and marks
+// the chunk staged; the calling thread issues chunks in order. Download: the calling thread waits
+// until chunk i - kSlots has been emptied, issues chunk i into the slot and records the event; a
+// worker waits for it and empties the slot. Workers take chunks in order, so the oldest open chunk
+// always has someone working on it and nobody waits for a later one. A chunk is 40 us of the link,
+// about what a sleeping thread takes to wake, so the waits poll and yield.
+#include "pct_stage.h"
+
+#include <string.h>
+
+#include <algorithm>
+#include <mutex>
+
+namespace pct {
+namespace {
+
+template <class F>
+void poll_until(F &&done) {
+  for (int i = 0; !done(); ++i)
+    if (i > 64) std::this_thread::yield();
+}
+
+// Pinned blocks that no stager holds, guarded by the mutex; freed with the last stager.
+struct Block {
+  int device;
+  char *slots;
+  cudaEvent_t ev[HostStager::kSlots];
+};
+constexpr size_t kMaxSpare = 2;
+std::mutex spare_mutex;
+std::vector<Block> spare;
+int stagers = 0;
+
+void free_block(const Block &b) {
+  for (cudaEvent_t e : b.ev)
+    if (e) cudaEventDestroy(e);
+  cudaFreeHost(b.slots);
+}
+
+}  // namespace
+
+HostStager::HostStager() {
+  std::lock_guard<std::mutex> lock(spare_mutex);
+  ++stagers;
+}
+
+HostStager::~HostStager() {
+  release();
+  std::lock_guard<std::mutex> lock(spare_mutex);
+  if (--stagers > 0) return;
+  for (const Block &b : spare) free_block(b);
+  spare.clear();
+}
+
+bool HostStager::pageable(const void *p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+int HostStager::worker_count() const {
+  const unsigned hw = std::thread::hardware_concurrency();
+  return (int)std::min(3u, std::max(1u, hw / 2));
+}
+
+bool HostStager::reserve(int device) {
+  if (slots_) return true;
+  device_ = device;
+  {
+    std::lock_guard<std::mutex> lock(spare_mutex);
+    for (size_t i = 0; i < spare.size(); ++i) {
+      if (spare[i].device != device) continue;
+      slots_ = spare[i].slots;
+      std::copy(spare[i].ev, spare[i].ev + kSlots, ev_);
+      spare.erase(spare.begin() + i);
+      return true;
+    }
+  }
+  if (cudaSetDevice(device) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void **>(&slots_), kSlots * kSlotBytes, cudaHostAllocDefault) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    slots_ = nullptr;
+    return false;
+  }
+  for (int k = 0; k < kSlots; ++k) {
+    used_[k] = false;
+    if (cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      release();
+      return false;
+    }
+  }
+  return true;
+}
+
+// Waits for the transfers of its own slots, then leaves them on the list or frees them.
+void HostStager::release() {
+  end();
+  if (!slots_) return;
+  Block b{device_, slots_, {}};
+  bool whole = true;
+  for (int k = 0; k < kSlots; ++k) {
+    if (used_[k] && cudaEventSynchronize(ev_[k]) != cudaSuccess) whole = false;
+    whole = whole && ev_[k];
+    b.ev[k] = ev_[k];
+    ev_[k] = nullptr;
+    used_[k] = false;
+  }
+  slots_ = nullptr;
+  std::lock_guard<std::mutex> lock(spare_mutex);
+  try {
+    if (whole && spare.size() < kMaxSpare) {
+      spare.push_back(b);
+      return;
+    }
+  } catch (...) {
+  }
+  free_block(b);
+}
+
+// Starts the workers on chunks_.
+bool HostStager::start(int device, bool uploads) {
+  job_ = chunk_ = 0;
+  issued_ = 0;
+  next_ = 0;
+  cancel_ = false;
+  error_ = (int)cudaSuccess;
+  try {
+    if (staged_size_ < chunks_.size()) {
+      staged_.reset(new std::atomic<char>[chunks_.size()]);
+      staged_size_ = chunks_.size();
+    }
+    for (size_t i = 0; i < chunks_.size(); ++i) staged_[i] = 0;
+    const int n = (int)std::min<size_t>(worker_count(), chunks_.size());
+    threads_.reserve(n);
+    for (int k = 0; k < n; ++k) threads_.emplace_back([this, device, uploads] { work(device, uploads); });
+  } catch (...) {
+    if (threads_.empty()) return false;  // (fewer workers than asked for are enough)
+  }
+  return true;
+}
+
+bool HostStager::begin(int device, const std::vector<Job> &jobs) {
+  end();
+  try {
+    size_t total = 0;
+    for (const Job &j : jobs) total += j.bytes;
+    if (total < kMinBytes) return false;
+    for (const Job &j : jobs)
+      if (!pageable(j.src)) return false;
+    if (!reserve(device)) return false;
+    chunks_.clear();
+    jobs_ = jobs;
+    for (const Job &j : jobs)
+      for (size_t o = 0; o < j.bytes; o += kSlotBytes)
+        chunks_.push_back(Chunk{static_cast<const char *>(j.src) + o, nullptr,
+                                std::min(kSlotBytes, j.bytes - o)});
+    return start(device, true);
+  } catch (...) {  // out of host memory
+    end();
+    return false;
+  }
+}
+
+void HostStager::work(int device, bool uploads) {
+  cudaError_t bad = cudaSetDevice(device);
+  for (;;) {
+    const size_t i = next_.fetch_add(1);
+    if (i >= chunks_.size()) return;
+    const int slot = (int)(i % kSlots);
+    char *mem = slots_ + slot * kSlotBytes;
+    const size_t need = uploads ? (i >= kSlots ? i - kSlots + 1 : 0) : i + 1;
+    poll_until([&] { return cancel_.load() || issued_.load(std::memory_order_acquire) >= need; });
+    if (cancel_) return;
+    // (uploads: also a transfer of an earlier call may still read the slot)
+    if (bad == cudaSuccess && (!uploads || used_[slot]))
+      poll_until([&] {
+        bad = cudaEventQuery(ev_[slot]);
+        return bad != cudaErrorNotReady || cancel_.load();
+      });
+    if (cancel_) return;
+    if (bad == cudaSuccess) {
+      const Chunk &c = chunks_[i];
+      if (uploads)
+        memcpy(mem, c.src, c.bytes);
+      else
+        memcpy(c.dst, mem, c.bytes);
+    }
+    if (bad != cudaSuccess) error_ = (int)bad;
+    staged_[i].store(1, std::memory_order_release);
+  }
+}
+
+cudaError_t HostStager::copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  if (!active() || job_ >= jobs_.size() || jobs_[job_].src != src || jobs_[job_].bytes != bytes)
+    return cudaErrorInvalidValue;
+  ++job_;
+  for (size_t o = 0; o < bytes; o += kSlotBytes, ++chunk_) {
+    const size_t i = chunk_;
+    const int slot = (int)(i % kSlots);
+    poll_until([&] { return staged_[i].load(std::memory_order_acquire) != 0; });
+    if (error_ != (int)cudaSuccess) return (cudaError_t)error_.load();
+    cudaError_t e = cudaMemcpyAsync(static_cast<char *>(dst) + o, slots_ + slot * kSlotBytes,
+                                    chunks_[i].bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaEventRecord(ev_[slot], s);
+    if (e != cudaSuccess) return e;
+    used_[slot] = true;
+    issued_.store(i + 1, std::memory_order_release);
+  }
+  return cudaSuccess;
+}
+
+void HostStager::end() {
+  cancel_ = true;
+  for (std::thread &t : threads_) t.join();
+  threads_.clear();
+}
+
+cudaError_t HostStager::download(int device, void *dst, const void *src, size_t bytes,
+                                 cudaStream_t s) {
+  end();
+  bool staged = bytes >= kMinBytes && pageable(dst) && reserve(device);
+  if (staged) {
+    try {
+      chunks_.clear();
+      jobs_.clear();
+      for (size_t o = 0; o < bytes; o += kSlotBytes)
+        chunks_.push_back(Chunk{static_cast<const char *>(src) + o, static_cast<char *>(dst) + o,
+                                std::min(kSlotBytes, bytes - o)});
+      staged = start(device, false);
+    } catch (...) {
+      end();
+      staged = false;
+    }
+  }
+  if (!staged) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+  }
+  cudaError_t e = cudaSuccess;
+  for (size_t i = 0; i < chunks_.size() && e == cudaSuccess; ++i) {
+    const int slot = (int)(i % kSlots);
+    if (i >= kSlots) poll_until([&] { return staged_[i - kSlots].load(std::memory_order_acquire) != 0; });
+    e = (cudaError_t)error_.load();
+    // (a slot's earlier upload runs before this on the device only if the streams are ordered)
+    if (e == cudaSuccess && i < kSlots && used_[slot]) e = cudaEventSynchronize(ev_[slot]);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(slots_ + slot * kSlotBytes, chunks_[i].src, chunks_[i].bytes,
+                          cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaEventRecord(ev_[slot], s);
+    if (e != cudaSuccess) break;
+    used_[slot] = true;
+    issued_.store(i + 1, std::memory_order_release);
+  }
+  if (e == cudaSuccess) {
+    for (size_t i = 0; i < chunks_.size(); ++i)
+      poll_until([&] { return staged_[i].load(std::memory_order_acquire) != 0; });
+    e = (cudaError_t)error_.load();
+  }
+  end();
+  return e;
+}
+
+}  // namespace pct
