@@ -305,10 +305,9 @@ int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in
       h->last_error.clear();
       return PCT_OK;
     }
-    PCT_CUDA(h, pct::launch_pitch_copy(in.atlas, static_cast<float *>(h->atlas.ptr), rows, g.ny,
-                                       pitch, s));
-    PCT_CUDA(h, pct::launch_pitch_copy(in.label, static_cast<float *>(h->label.ptr), rows, g.ny,
-                                       pitch, s));
+    PCT_CUDA(h, pct::launch_pitch_copy_pair(in.atlas, static_cast<float *>(h->atlas.ptr), in.label,
+                                            static_cast<float *>(h->label.ptr), rows, g.ny, pitch,
+                                            s));
     in = pct::SlabInputs{in.img, static_cast<const float *>(h->atlas.ptr),
                          static_cast<const float *>(h->label.ptr), pitch};
   }
@@ -1057,10 +1056,9 @@ int pct_synthesize_device(pct_handle *h, const float *d_img, const float *d_atla
     const long long rows = (long long)g.num * g.nz * g.nx;
     const size_t bytes = (size_t)rows * pitch * sizeof(float);
     if ((st = ensure(h, h->atlas, bytes)) || (st = ensure(h, h->label, bytes))) return st;
-    PCT_CUDA(h, pct::launch_pitch_copy(d_atlas, static_cast<float *>(h->atlas.ptr), rows, g.ny,
-                                       pitch, s));
-    PCT_CUDA(h, pct::launch_pitch_copy(d_atlas_label, static_cast<float *>(h->label.ptr), rows,
-                                       g.ny, pitch, s));
+    PCT_CUDA(h, pct::launch_pitch_copy_pair(d_atlas, static_cast<float *>(h->atlas.ptr),
+                                            d_atlas_label, static_cast<float *>(h->label.ptr), rows,
+                                            g.ny, pitch, s));
     in = pct::SlabInputs{d_img, static_cast<const float *>(h->atlas.ptr),
                          static_cast<const float *>(h->label.ptr), pitch};
   }
@@ -1161,7 +1159,7 @@ int pct_query_plan(int device, int nx, int ny, int nz, int num_atlas, int nh, pc
   plan->tile_rows = info.rx;
   plan->tile_planes = info.tz;
   plan->scratch_bytes = info.partial_bytes;
-  plan->launches = work ? 1 + (ny % 4 != 0 ? 2 : 0) + (info.groups > 1 ? 1 : 0) : 0;
+  plan->launches = work ? 1 + (ny % 4 != 0 ? 1 : 0) + (info.groups > 1 ? 1 : 0) : 0;
   return PCT_OK;
 }
 
@@ -1404,8 +1402,7 @@ int stage_batch(pct_handle *h, const pct_subject *subs, int n, const std::vector
       float *a = reinterpret_cast<float *>(p);
       float *l = reinterpret_cast<float *>(p + bytes);
       p += 2 * bytes + 256 - (2 * bytes) % 256;
-      PCT_CUDA(h, pct::launch_pitch_copy(sb.atlas, a, rows, sb.ny, pitch, s));
-      PCT_CUDA(h, pct::launch_pitch_copy(sb.atlas_label, l, rows, sb.ny, pitch, s));
+      PCT_CUDA(h, pct::launch_pitch_copy_pair(sb.atlas, a, sb.atlas_label, l, rows, sb.ny, pitch, s));
       si = pct::SlabInputs{sb.img, a, l, pitch};
     }
     in[i] = pct::BatchSubjectIn{geo[i], si, sb.out, sb.div};

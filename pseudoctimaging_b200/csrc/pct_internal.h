@@ -147,6 +147,9 @@ cudaError_t launch_prepared_batch(const BatchSetup &setup, cudaStream_t stream);
 // dst[r*pitch + c] = src[r*ny + c] for r < rows, c < ny.
 cudaError_t launch_pitch_copy(const float *src, float *dst, long long rows, int ny, int pitch,
                               cudaStream_t stream);
+// The same for two stacks of one shape in one launch.
+cudaError_t launch_pitch_copy_pair(const float *src0, float *dst0, const float *src1, float *dst1,
+                                   long long rows, int ny, int pitch, cudaStream_t stream);
 
 inline int slab_pitch(int ny) { return (ny + 3) / 4 * 4; }
 
