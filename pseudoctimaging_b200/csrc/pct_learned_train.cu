@@ -101,7 +101,7 @@ __global__ void targets_kernel(const SubjectRef *__restrict__ subs, const int *_
 //    multiply-adds per row); nine warps take conv2 while the other three take conv3.
 // The gradient of conv1's output overwrites that output, and conv3's likewise, once the weight
 // gradients that read it are done. 4,096 samples: 13.8 ms with one output per thread and the
-// gradients in shared memory, 1.33 ms now (gradients read back, whole call).
+// gradients in shared memory, 1.21 ms now (gradients read back, whole call).
 
 constexpr int kTS = 3;  // samples per CTA pass: what fits beside the weights in 227 KB
 
@@ -197,15 +197,32 @@ __device__ __forceinline__ void grad_row(const float (&w)[27][kC][kC], const flo
 #pragma unroll
         for (int y = 0; y < SO; ++y) v[y] = ld4(row + y * kC);
 #pragma unroll
-        for (int ky = 0; ky < 3; ++ky)
+        for (int ky = 0; ky < 3; ++ky) {
+          float4 wv[4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 wv = ld4(&w[(kz * 3 + kx) * 3 + ky][4 * cg + c][wgroup(4 * cg, g)]);
+          for (int c = 0; c < 4; ++c)
+            wv[c] = ld4(&w[(kz * 3 + kx) * 3 + ky][4 * cg + c][wgroup(4 * cg, g)]);
+          // (four multiply-adds in a row share one operand: three fresh ones each take 1.6 cycles)
 #pragma unroll
-            for (int y = 0; y < SO; ++y) acc[y + ky][c] = dot(wv, v[y], acc[y + ky][c]);
-          }
+          for (int y = 0; y < SO; ++y)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                acc[y + ky][c] = fmaf(get(v[y], k), get(wv[c], k), acc[y + ky][c]);
+        }
       }
 }
+
+// Rows (z * SI + x) of the input-gradient phases by how many (kz, kx) reach them, 9 first: a warp's
+// lanes then take the same number of steps, and the long warps spread over the schedulers. (In
+// plain order every warp held a row with the longest loops: conv2's phase was 31 % of the whole
+// pass; 4,096 samples 1.33 ms, 1.23 with the order.)
+__constant__ unsigned char kRowOrder7[49] = {
+    16, 17, 18, 23, 24, 25, 30, 31, 32, 15, 19, 22, 26, 29, 33, 9, 10, 11, 37, 38, 39, 8, 12, 36, 40,
+    14, 20, 21, 27, 28, 34, 2, 3, 4, 44, 45, 46, 7, 13, 35, 41, 1, 5, 43, 47, 0, 6, 42, 48};
+__constant__ unsigned char kRowOrder5[25] = {
+    12, 11, 13, 7, 17, 6, 8, 16, 18, 10, 14, 2, 22, 5, 9, 15, 19, 1, 3, 21, 23, 0, 4, 20, 24};
 
 // Adds one sample's share of the weight gradients of one (kz, kx): acc[ky][2 co][4 ci] of the
 // lane's co pair and ci group.
@@ -227,11 +244,10 @@ __device__ __forceinline__ void weight_rows(const float *in, const float *dz, in
 #pragma unroll
       for (int ky = 0; ky < 3; ++ky)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float a = get(v[y + ky], c);
-          acc[ky * 8 + c] = fmaf(d.x, a, acc[ky * 8 + c]);
-          acc[ky * 8 + 4 + c] = fmaf(d.y, a, acc[ky * 8 + 4 + c]);
-        }
+        for (int o = 0; o < 2; ++o)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            acc[ky * 8 + o * 4 + c] = fmaf(o ? d.y : d.x, get(v[y + ky], c), acc[ky * 8 + o * 4 + c]);
     }
   }
 }
@@ -449,7 +465,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     __syncthreads();
     // conv3's input gradient
     if (tid < ns * 25 * 4) {
-      const int cg = tid & 3, si = (tid >> 2) / 25, row = (tid >> 2) % 25;
+      const int cg = tid & 3, si = (tid >> 2) % ns, row = kRowOrder5[(tid >> 2) / ns];
       float acc[5][4];
       grad_row<5, 3>(S.w[1], S.s[si].a3, row / 5, row % 5, cg, acc);
 #pragma unroll
@@ -477,7 +493,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     __syncthreads();
     // conv2's input gradient, over conv1's output
     for (int t = tid; t < ns * 49 * 4; t += kTrainThreads) {
-      const int cg = t & 3, si = (t >> 2) / 49, row = (t >> 2) % 49;
+      const int cg = t & 3, si = (t >> 2) % ns, row = kRowOrder7[(t >> 2) / ns];
       float acc[7][4];
       grad_row<7, 5>(S.w[0], S.s[si].d2, row / 7, row % 7, cg, acc);
 #pragma unroll
