@@ -1235,9 +1235,12 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
   cudaStream_t s = h->user_stream ? h->user_stream : h->stream;
   float *d_img = static_cast<float *>(h->img.ptr), *d_out = static_cast<float *>(h->out.ptr);
   PCT_CUDA(h, cudaMemsetAsync(d_out, 0, vol, s));
+  // (the fused volume itself is downloaded by plane ranges, as pct_synthesize does)
+  float *const by_ranges = regularize ? nullptr : out;
   st = uses_tma_rows(exec_choice)
-           ? fuse_pipelined(h, g, img, atlas_mri, atlas_ct_hu, d_out, div, true, nullptr, s)
+           ? fuse_pipelined(h, g, img, atlas_mri, atlas_ct_hu, d_out, div, true, by_ranges, s)
            : PCT_ERR_UNSUPPORTED;
+  const bool downloaded = st == PCT_OK && by_ranges;
   if (st == PCT_ERR_UNSUPPORTED) {  // one upload, then the path
     h->last_error.clear();
     StageScope staging{h->stager};
@@ -1264,7 +1267,7 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
     PCT_CUDA(h, pct::launch_regularize(d_out, nx, ny, nz, nh, h->scratch.ptr, s, &f, &rounds));
     PCT_CUDA(h, pct::launch_finalize_hu(d_out, (size_t)g.nvox(), s));
   }
-  PCT_CUDA(h, download(h, out, d_out, vol, s));
+  if (!downloaded) PCT_CUDA(h, download(h, out, d_out, vol, s));
   PCT_CUDA(h, cudaStreamSynchronize(s));
   return PCT_OK;
 }
