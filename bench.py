@@ -468,11 +468,17 @@ def run_b200_arm(args) -> None:
     if world > 1:
         dist.destroy_process_group()
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        r = cpu_reference_rate(args.cpu_seconds)
-        cpu_value = nvox / (cand / r["cand_per_s"])
-        line["cpu_baseline"] = {"value": cpu_value, "unit": UNIT, "cores": r["cores"],
-                                "kind": "reference", "sample": r["sample"],
-                                "seconds": r["seconds"], "cand_per_s": r["cand_per_s"]}
+        import oracle
+
+        if oracle.has_reference():
+            r = cpu_reference_rate(args.cpu_seconds)
+            cpu_value = nvox / (cand / r["cand_per_s"])
+            line["cpu_baseline"] = {"value": cpu_value, "unit": UNIT, "cores": r["cores"],
+                                    "kind": "reference", "sample": r["sample"],
+                                    "seconds": r["seconds"], "cand_per_s": r["cand_per_s"]}
+        else:  # built only where the reference's sources are
+            line["cpu_baseline"] = {"unavailable": "oracle/_ref/libpctref.so was not built "
+                                                   "(reference sources absent at build time)"}
     if rank == 0:
         print(json.dumps(line))
 

@@ -67,3 +67,29 @@ def test_cap_and_capture_keep_to_the_scratch_there_is():
         torch.cuda.synchronize()
         h.device_status()
         compare_fused(out.cpu().numpy(), ref, nh, 1e-4, prod, sumw)
+
+
+def test_capture_after_a_warm_up_replays_the_same_plan():
+    """A captured call whose scratch is there keeps its groups and their combine: the replay equals
+    the direct call bit for bit, on new inputs in the same buffers too."""
+    nx, ny, nz, num, nh = 40, 43, 26, 2, 9  # ny % 4 != 0: the repack is captured as well
+    div = pct.div_from(2.5, 1.0)
+    subs = [pct.synth_subject(nx, ny, nz, num, n_blobs=6, seed=k) for k in (6, 7)]
+    labs = [pct.normalize_labels(s.atlas_ct) for s in subs]
+    assert pct.query_plan(nx, ny, nz, num, nh)["groups"] > 1
+    with pct.Handle(0) as h:
+        ref = [run(h, s, lab, nh, div) for s, lab in zip(subs, labs)]
+        d = [torch.empty(a.shape, device="cuda") for a in (subs[0].img, subs[0].atlas_mri, labs[0])]
+        out = torch.zeros_like(d[0])
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            h.synthesize_device(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), out.data_ptr(),
+                                nx, ny, nz, num, nh, div, pct.EXEC_B200_FP32,
+                                torch.cuda.current_stream().cuda_stream)
+        for s, lab, r in zip(subs, labs, ref):
+            for t, a in zip(d, (s.img, s.atlas_mri, lab)):
+                t.copy_(torch.from_numpy(np.ascontiguousarray(a)))
+            g.replay()
+            torch.cuda.synchronize()
+            h.device_status()
+            np.testing.assert_array_equal(out.cpu().numpy(), r)
