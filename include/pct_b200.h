@@ -113,13 +113,14 @@ int pct_device_status(pct_handle *h, void *stream);
 
 /*
  * How pct_synthesize_device would run a given shape on `device` (no work is done): the kernel
- * launches it issues (fusion, pitched repack copies when ny % 4 != 0 or buffers are not 16-byte
- * aligned — assumed aligned here —, the atlas-group combine), the number of atlas groups, the
+ * launches it issues (fusion, one pitched repack of both stacks when ny % 4 != 0 or buffers are not
+ * 16-byte aligned — assumed aligned here —, the group combine), the number of groups (atlas groups
+ * times the ranges that a small volume's window is split into; no memory cap assumed), the
  * register tile and the persistent grid.
  */
 typedef struct pct_plan {
   int launches;        /* kernel launches per call */
-  int groups;          /* atlas groups (work items per tile) */
+  int groups;          /* groups (work items per tile) */
   int tiles;           /* output tiles */
   int ctas;            /* persistent CTAs launched */
   int tile_rows;       /* RX: x rows per warp */
