@@ -93,22 +93,24 @@ __global__ void targets_kernel(const SubjectRef *__restrict__ subs, const int *_
 // so every phase works on a register tile that uses each value it loads several times. A CTA of 12
 // warps takes kTS samples at a time; activations are channels-last ([position][16]), weights
 // [tap][ci][co], so that four channels are one 16-byte load:
-//  * forward and input gradients: a thread owns one output row along y and four channels; a (kz,
-//    kx, four channels) step loads the input row once for its three y taps (conv2: 19 loads for
-//    240 multiply-adds);
+//  * forward and input gradients: a thread owns one output row along y and four channels; a step
+//    loads the input row once for its three y taps. The forward sums start at the bias and run over
+//    input channels, then taps, one after the other: a pre-activation near zero changes its side of
+//    the ReLU with the order of its sum, and one of those moves the gradient by 1e-6. (Channels in
+//    groups of four, conv3 and conv4 in partial sums: 1.21 ms, and other sides taken.)
 //  * weight gradients: a warp owns the 16 x 16 x 3 (co, ci, ky) weights of one (kz, kx), 24 per
 //    lane, and keeps their sums in registers over all samples of the CTA (conv2: 12 loads for 120
 //    multiply-adds per row); nine warps take conv2 while the other three take conv3.
 // The gradient of conv1's output overwrites that output, and conv3's likewise, once the weight
 // gradients that read it are done. 4,096 samples: 13.8 ms with one output per thread and the
-// gradients in shared memory, 1.21 ms now (gradients read back, whole call).
+// gradients in shared memory, 1.28 ms now (gradients read back, whole call).
 
 constexpr int kTS = 3;  // samples per CTA pass: what fits beside the weights in 227 KB
 
 struct SampleSmem {
   float x0[kCin * kNX + 2];  // scaled input patches [ci][z][x][y]
-  float a1[kN1 * kC];        // conv1's output, later its gradient ([position][channel])
-  float a2[kN2 * kC];
+  float a1[kN1 * kC];        // conv1's output, later its gradient ([position][channel], rotated)
+  float a2[kN2 * kC];        // (rotated as well)
   float a3[kN3 * kC];        // conv3's output, later its gradient
   float d2[kN2 * kC];
   float a4[kC], d4[kC];
@@ -123,7 +125,6 @@ struct TrainSmem {
   __align__(16) float small[kSmall];   // biases [4][16], heads [33][16], head biases [33]
   __align__(16) float gsmall[kSmall];  // this CTA's gradient sums of the same
   __align__(16) SampleSmem s[kTS];
-  float part4[kTS][8][kC];
   float loss;
 };
 static_assert(sizeof(TrainSmem) <= 227 * 1024, "shared memory");
@@ -152,28 +153,33 @@ __device__ __forceinline__ float dot(const float4 &a, const float4 &b, float acc
 // half of all shared wavefronts were conflicts, 1.62 ms for the 4,096 samples.)
 __device__ __forceinline__ int wgroup(int ci, int cog) { return 4 * (cog ^ (ci >> 2)); }
 
+// Place of channel group g in row `row` (z * S + x) of a1 and a2: rotated by the row, so that lanes on
+// consecutive rows that read one channel (forward) hit different banks.
+__device__ __forceinline__ int agroup(int row, int g) { return 4 * (g ^ ((row >> 1) & 3)); }
+
 // One output row (SO positions along y, row (z, x)) and channels [4 cg, 4 cg + 4) of a 16 -> 16
-// convolution, over the input channel groups [g0, g1).
+// convolution, added to acc in the order of the input channels and, within one, of the taps.
 template <int SI, int SO>
 __device__ __forceinline__ void conv_row(const float (&w)[27][kC][kC], const float *in, int z, int x,
-                                         int cg, int g0, int g1, float (&acc)[SO][4]) {
+                                         int cg, float (&acc)[SO][4]) {
 #pragma unroll 1
-  for (int g = g0; g < g1; ++g)
-#pragma unroll 1
+  for (int ci = 0; ci < kC; ++ci) {
+    const int wg = wgroup(ci, cg);
+#pragma unroll 3
     for (int kzx = 0; kzx < 9; ++kzx) {
-      const float *row = in + ((z + kzx / 3) * SI + x + kzx % 3) * SI * kC + 4 * g;
-      float4 v[SO + 2];
+      const int r = (z + kzx / 3) * SI + x + kzx % 3;
+      const float *row = in + r * SI * kC + agroup(r, ci >> 2) + (ci & 3);
+      float v[SO + 2];
 #pragma unroll
-      for (int y = 0; y < SO + 2; ++y) v[y] = ld4(row + y * kC);
+      for (int y = 0; y < SO + 2; ++y) v[y] = row[y * kC];
 #pragma unroll
-      for (int ky = 0; ky < 3; ++ky)
+      for (int ky = 0; ky < 3; ++ky) {
+        const float4 wv = ld4(&w[kzx * 3 + ky][ci][wg]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float4 wv = ld4(&w[kzx * 3 + ky][4 * g + c][wgroup(4 * g, cg)]);
-#pragma unroll
-          for (int y = 0; y < SO; ++y) axpy(acc[y], get(v[y + ky], c), wv);
-        }
+        for (int y = 0; y < SO; ++y) axpy(acc[y], v[y + ky], wv);
+      }
     }
+  }
 }
 
 // One input row (SI positions along y, row (z, x)) and input channels [4 cg, 4 cg + 4) of the
@@ -229,11 +235,12 @@ __constant__ unsigned char kRowOrder5[25] = {
 template <int SI, int SO>
 __device__ __forceinline__ void weight_rows(const float *in, const float *dz, int kz, int kx, int lane,
                                             float *acc) {
-  const int cop = 2 * (lane >> 2), cig = 4 * (lane & 3);
+  const int cop = 2 * (lane >> 2), cig = lane & 3;
 #pragma unroll 1
   for (int r = 0; r < SO * SO; ++r) {
     const int z = r / SO, x = r - z * SO;
-    const float *row = in + ((z + kz) * SI + x + kx) * SI * kC + cig;
+    const int ri = (z + kz) * SI + x + kx;
+    const float *row = in + ri * SI * kC + agroup(ri, cig);
     const float *drow = dz + r * SO * kC + cop;
     float4 v[SO + 2];
 #pragma unroll
@@ -338,7 +345,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           for (int y = 0; y < 7; ++y) axpy(acc[y], v[y + ky], wv);
         }
       }
-      float *dst = S.s[si].a1 + row * 7 * kC + 4 * cg;
+      float *dst = S.s[si].a1 + row * 7 * kC + agroup(row, cg);
 #pragma unroll
       for (int y = 0; y < 7; ++y)
         *reinterpret_cast<float4 *>(dst + y * kC) =
@@ -353,8 +360,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       const float4 b = ld4(S.small + kSmallB + kC + 4 * cg);
 #pragma unroll
       for (int y = 0; y < 5; ++y) acc[y][0] = b.x, acc[y][1] = b.y, acc[y][2] = b.z, acc[y][3] = b.w;
-      conv_row<7, 5>(S.w[0], S.s[si].a1, row / 5, row % 5, cg, 0, 4, acc);
-      float *dst = S.s[si].a2 + row * 5 * kC + 4 * cg;
+      conv_row<7, 5>(S.w[0], S.s[si].a1, row / 5, row % 5, cg, acc);
+      float *dst = S.s[si].a2 + row * 5 * kC + agroup(row, cg);
 #pragma unroll
       for (int y = 0; y < 5; ++y)
         *reinterpret_cast<float4 *>(dst + y * kC) =
@@ -362,44 +369,29 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                         fmaxf(acc[y][3], 0.f));
     }
     __syncthreads();
-    // conv3: two threads share an output, each half of the input channels
-    {
-      const bool on = tid < ns * 9 * 4 * 2;
-      const int half = tid & 1, cg = (tid >> 1) & 3, r = on ? tid >> 3 : 0, si = r / 9, row = r % 9;
+    // conv3
+    if (tid < ns * 9 * 4) {
+      const int cg = tid & 3, si = (tid >> 2) / 9, row = (tid >> 2) % 9;
       float acc[3][4];
-#pragma unroll
-      for (int y = 0; y < 3; ++y)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[y][c] = 0.f;
-      if (on) conv_row<5, 3>(S.w[1], S.s[si].a2, row / 3, row % 3, cg, 2 * half, 2 * half + 2, acc);
       const float4 b = ld4(S.small + kSmallB + 2 * kC + 4 * cg);
 #pragma unroll
-      for (int y = 0; y < 3; ++y) {
+      for (int y = 0; y < 3; ++y) acc[y][0] = b.x, acc[y][1] = b.y, acc[y][2] = b.z, acc[y][3] = b.w;
+      conv_row<5, 3>(S.w[1], S.s[si].a2, row / 3, row % 3, cg, acc);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[y][c] += __shfl_xor_sync(0xffffffffu, acc[y][c], 1);
-        if (on && half == 0)
-          *reinterpret_cast<float4 *>(S.s[si].a3 + (row * 3 + y) * kC + 4 * cg) =
-              make_float4(fmaxf(acc[y][0] + b.x, 0.f), fmaxf(acc[y][1] + b.y, 0.f),
-                          fmaxf(acc[y][2] + b.z, 0.f), fmaxf(acc[y][3] + b.w, 0.f));
-      }
+      for (int y = 0; y < 3; ++y)
+        *reinterpret_cast<float4 *>(S.s[si].a3 + (row * 3 + y) * kC + 4 * cg) =
+            make_float4(fmaxf(acc[y][0], 0.f), fmaxf(acc[y][1], 0.f), fmaxf(acc[y][2], 0.f),
+                        fmaxf(acc[y][3], 0.f));
     }
     __syncthreads();
-    // conv4: the 432-term sums in eight parts
-    {
-      const int si = tid >> 7, part = (tid >> 4) & 7, co = tid & 15;
-      if (si < ns) {
-        const float *w4 = &S.w[2][0][0][0];
-        float acc = 0.f;
-#pragma unroll 6
-        for (int q = part; q < 27 * kC; q += 8) acc = fmaf(w4[q * kC + co], S.s[si].a3[q], acc);
-        S.part4[si][part][co] = acc;
-      }
-    }
-    __syncthreads();
+    // conv4
     if (tid < ns * kC) {
       const int si = tid / kC, co = tid % kC;
+      const float *w4 = &S.w[2][0][0][0], *a3 = S.s[si].a3;
       float acc = S.small[kSmallB + 3 * kC + co];
-      for (int q = 0; q < 8; ++q) acc += S.part4[si][q][co];
+      for (int ci = 0; ci < kC; ++ci)
+#pragma unroll
+        for (int k = 0; k < 27; ++k) acc = fmaf(w4[(k * kC + ci) * kC + co], a3[k * kC + ci], acc);
       S.s[si].a4[co] = fmaxf(acc, 0.f);
     }
     __syncthreads();
@@ -470,9 +462,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       grad_row<5, 3>(S.w[1], S.s[si].a3, row / 5, row % 5, cg, acc);
 #pragma unroll
       for (int y = 0; y < 5; ++y) {
-        const int at = (row * 5 + y) * kC + 4 * cg;
-        const float4 a = ld4(S.s[si].a2 + at);
-        *reinterpret_cast<float4 *>(S.s[si].d2 + at) =
+        const float4 a = ld4(S.s[si].a2 + (row * 5 + y) * kC + agroup(row, cg));
+        *reinterpret_cast<float4 *>(S.s[si].d2 + (row * 5 + y) * kC + 4 * cg) =
             make_float4(a.x > 0.f ? acc[y][0] : 0.f, a.y > 0.f ? acc[y][1] : 0.f,
                         a.z > 0.f ? acc[y][2] : 0.f, a.w > 0.f ? acc[y][3] : 0.f);
       }
@@ -498,7 +489,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       grad_row<7, 5>(S.w[0], S.s[si].d2, row / 7, row % 7, cg, acc);
 #pragma unroll
       for (int y = 0; y < 7; ++y) {
-        float4 *a1 = reinterpret_cast<float4 *>(S.s[si].a1 + (row * 7 + y) * kC + 4 * cg);
+        float4 *a1 =
+            reinterpret_cast<float4 *>(S.s[si].a1 + (row * 7 + y) * kC + agroup(row, cg));
         const float4 a = *a1;
         *a1 = make_float4(a.x > 0.f ? acc[y][0] : 0.f, a.y > 0.f ? acc[y][1] : 0.f,
                           a.z > 0.f ? acc[y][2] : 0.f, a.w > 0.f ? acc[y][3] : 0.f);
@@ -507,7 +499,6 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     __syncthreads();
     // conv1's weight gradients: a warp's two (ci, kz, kx), lanes over rows and channel groups
     if (warp < 9) {
-      const int cg = 4 * (lane & 3);
       for (int si = 0; si < ns; ++si)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -520,7 +511,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             for (int y = 0; y < 9; ++y) v[y] = src[y];
 #pragma unroll
             for (int y = 0; y < 7; ++y) {
-              const float4 d = ld4(S.s[si].a1 + (row * 7 + y) * kC + cg);
+              const float4 d = ld4(S.s[si].a1 + (row * 7 + y) * kC + agroup(row, lane & 3));
 #pragma unroll
               for (int ky = 0; ky < 3; ++ky)
 #pragma unroll
@@ -534,7 +525,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       // (three warps may add to the same channels: one sample each)
       float acc = 0.f;
       const float *d = S.s[warp - 9].a1;
-      for (int p = lane >> 4; p < kN1; p += 2) acc += d[p * kC + (lane & 15)];
+      for (int p = lane >> 4; p < kN1; p += 2)
+        acc += d[p * kC + agroup(p / 7, (lane & 15) >> 2) + (lane & 3)];
       acc += __shfl_xor_sync(0xffffffffu, acc, 16);
       if (lane < kC) atomicAdd(S.gsmall + kSmallB + lane, acc);
     }
