@@ -7,7 +7,9 @@
 // about what a sleeping thread takes to wake, so the waits poll and yield.
 #include "pct_stage.h"
 
+#include <stdint.h>
 #include <string.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <mutex>
@@ -32,10 +34,32 @@ std::mutex spare_mutex;
 std::vector<Block> spare;
 int stagers = 0;
 
+constexpr size_t kHuge = 2u << 20, kBlockBytes = HostStager::kSlots * HostStager::kSlotBytes;
+
+// kBlockBytes of host memory registered with the current device; nullptr if it cannot be had. Not
+// inherited by a fork: pages shared with a child would be copied away from the registration.
+char *pin_block() {
+  char *map = static_cast<char *>(mmap(nullptr, kBlockBytes + kHuge, PROT_READ | PROT_WRITE,
+                                       MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+  if (map == MAP_FAILED) return nullptr;
+  const size_t lead = (kHuge - reinterpret_cast<uintptr_t>(map) % kHuge) % kHuge;
+  char *p = map + lead;
+  if (lead) munmap(map, lead);
+  if (kHuge - lead) munmap(p + kBlockBytes, kHuge - lead);
+  madvise(p, kBlockBytes, MADV_HUGEPAGE);
+  if (madvise(p, kBlockBytes, MADV_DONTFORK) == 0 &&
+      cudaHostRegister(p, kBlockBytes, cudaHostRegisterDefault) == cudaSuccess)
+    return p;
+  cudaGetLastError();
+  munmap(p, kBlockBytes);
+  return nullptr;
+}
+
 void free_block(const Block &b) {
   for (cudaEvent_t e : b.ev)
     if (e) cudaEventDestroy(e);
-  cudaFreeHost(b.slots);
+  cudaHostUnregister(b.slots);
+  munmap(b.slots, kBlockBytes);
 }
 
 }  // namespace
@@ -67,7 +91,7 @@ int HostStager::worker_count() const {
   return (int)std::min(3u, std::max(1u, hw / 2));
 }
 
-bool HostStager::reserve(int device) {
+bool HostStager::reserve(int device, size_t bytes) {
   if (slots_) return true;
   device_ = device;
   {
@@ -80,13 +104,14 @@ bool HostStager::reserve(int device) {
       return true;
     }
   }
-  if (cudaSetDevice(device) != cudaSuccess ||
-      cudaHostAlloc(reinterpret_cast<void **>(&slots_), kSlots * kSlotBytes, cudaHostAllocDefault) !=
-          cudaSuccess) {
+  asked_ += bytes;
+  if (asked_ < kPinBytes) return false;
+  if (cudaSetDevice(device) != cudaSuccess) {
     cudaGetLastError();
-    slots_ = nullptr;
     return false;
   }
+  slots_ = pin_block();
+  if (!slots_) return false;
   for (int k = 0; k < kSlots; ++k) {
     used_[k] = false;
     if (cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming) != cudaSuccess) {
@@ -153,7 +178,7 @@ bool HostStager::begin(int device, const std::vector<Job> &jobs) {
     if (total < kMinBytes) return false;
     for (const Job &j : jobs)
       if (!pageable(j.src)) return false;
-    if (!reserve(device)) return false;
+    if (!reserve(device, total)) return false;
     chunks_.clear();
     jobs_ = jobs;
     for (const Job &j : jobs)
@@ -224,7 +249,7 @@ void HostStager::end() {
 cudaError_t HostStager::download(int device, void *dst, const void *src, size_t bytes,
                                  cudaStream_t s) {
   end();
-  bool staged = bytes >= kMinBytes && pageable(dst) && reserve(device);
+  bool staged = bytes >= kMinBytes && pageable(dst) && reserve(device, bytes);
   if (staged) {
     try {
       chunks_.clear();

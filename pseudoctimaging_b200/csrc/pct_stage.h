@@ -34,7 +34,8 @@ class HostStager {
   static bool pageable(const void *p);
 
   // Starts staging `jobs` in order. False (nothing started, the caller copies directly) when they are
-  // too small to gain, or the pinned slots or threads cannot be had.
+  // too small to gain, no slots are at hand and too little was copied yet to pin some, or the slots
+  // or threads cannot be had.
   bool begin(int device, const std::vector<Job> &jobs);
   bool active() const { return !threads_.empty(); }
   // The next job's transfer, enqueued on s. Jobs must be taken in the order given to begin.
@@ -52,6 +53,10 @@ class HostStager {
   static constexpr int kSlots = 8;
   static constexpr size_t kSlotBytes = 2u << 20;
   static constexpr size_t kMinBytes = 12u << 20;  // below, thread start and hand-over eat the gain
+  // A stager without slots copies directly until it has been asked for this much: pinning slots takes
+  // 2.6 ms and staging gains 0.04 to 0.065 ms per MB, so a handle that makes one small call pays
+  // nothing for slots and one that stays pays at most about as much again as they cost.
+  static constexpr size_t kPinBytes = 60u << 20;
 
  private:
   struct Chunk {
@@ -59,9 +64,11 @@ class HostStager {
     char *dst;
     size_t bytes;
   };
-  // The slots come from a process-wide list of at most two blocks that stagers leave behind (pinning
-  // 16 MB takes about 20 ms) and go back to it; the last stager frees the list.
-  bool reserve(int device);
+  // The slots come from a process-wide list of at most two blocks that stagers leave behind and go
+  // back to it; the last stager frees the list. Slots are huge pages registered with the device: 2.6
+  // ms for 16 MB, where cudaHostAlloc takes 8 to 20 (a new handle's first call on 21 MB of arrays
+  // took 17 ms with it, 4.9 with direct copies as now).
+  bool reserve(int device, size_t bytes);
   void release();
   bool start(int device, bool uploads);
   void work(int device, bool uploads);
@@ -69,6 +76,7 @@ class HostStager {
 
   int device_ = -1;
   char *slots_ = nullptr;
+  size_t asked_ = 0;  // bytes that would have been staged while there were no slots
   cudaEvent_t ev_[kSlots] = {};
   bool used_[kSlots] = {};  // a transfer was recorded on ev_[k]
 

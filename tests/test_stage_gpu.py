@@ -87,3 +87,21 @@ def test_slots_pass_from_handle_to_handle():
         hs[3].close()
     for o in outs[1:]:
         np.testing.assert_array_equal(o, outs[0])
+
+
+@pytest.mark.parametrize("ny,calls", [(141, 3), (212, 2)])
+def test_slots_once_enough_was_copied(ny, calls):
+    """41 MB calls copy directly first and through slots later, 62 MB calls through slots at once, on
+    handles that come and go: the same volumes throughout."""
+    v = volumes(136, ny, 60, 4, ny)
+    with pct.Handle(0) as h:
+        ref = call(h, [t.pin_memory() for t in v], 3, pct.EXEC_B200_FP32, False)
+    for _ in range(2):
+        a, b = pct.Handle(0), pct.Handle(0)
+        for _ in range(calls):
+            for h in (a, b):
+                np.testing.assert_array_equal(call(h, v, 3, pct.EXEC_B200_FP32, False), ref)
+        a.close()  # its slots go to the next handle
+        with pct.Handle(0) as h:
+            np.testing.assert_array_equal(call(h, v, 3, pct.EXEC_B200_FP32, False), ref)
+        b.close()
