@@ -60,9 +60,9 @@ __global__ void collect_nan_kernel(const float *__restrict__ vol, int nx, int ny
 
 // One look at NaN voxel k by a whole warp: fills it if it is ready. Median() of the reference:
 // stable order of the non-NaN values among the 27 in (z, x, y) order, the middle one or the double
-// average of the two middle ones. Here each value's place in that order is counted. Returns
-// whether the voxel was filled.
-__device__ __forceinline__ bool try_fill(float *vol, int nx, int ny, int nz, int lo, int k, int lane) {
+// average of the two middle ones. Here each value's place in that order is counted.
+enum Look { kWaits, kFilled, kNanMedian };  // kNanMedian: ready, but the average of both infinities
+__device__ __forceinline__ Look try_fill(float *vol, int nx, int ny, int nz, int lo, int k, int lane) {
   const int nxy = nx * ny;
   const int z = k / nxy, x = k % nxy / ny, y = k % ny;
   const int dz = lane / 9 - 1, dx = lane / 3 % 3 - 1, dy = lane % 3 - 1;
@@ -73,10 +73,10 @@ __device__ __forceinline__ bool try_fill(float *vol, int nx, int ny, int nz, int
   // filled by the reference; they only drop out of the median.)
   const bool pending = nan && lane < 13 && z + dz >= lo && z + dz < nz - lo && x + dx >= lo &&
                        x + dx < nx - lo && y + dy >= lo && y + dy < ny - lo;
-  if (__any_sync(0xffffffffu, pending)) return false;
+  if (__any_sync(0xffffffffu, pending)) return kWaits;
   const unsigned have = __ballot_sync(0xffffffffu, on && !nan);
   const int cnt = __popc(have);
-  if (cnt == 0) return false;
+  if (cnt == 0) return kWaits;
   int rank = 0;
 #pragma unroll
   for (int j = 0; j < 27; ++j) {
@@ -89,8 +89,9 @@ __device__ __forceinline__ bool try_fill(float *vol, int nx, int ny, int nz, int
   const float b = __shfl_sync(0xffffffffu, v, __ffs(hi) - 1);
   const float a = __shfl_sync(0xffffffffu, v, low ? __ffs(low) - 1 : 0);
   const float m = (cnt & 1) == 0 ? (float)(((double)a + (double)b) / 2.0) : b;
+  if (isnan(m)) return kNanMedian;
   if (lane == 0) *((volatile float *)vol + k) = m;
-  return true;
+  return kFilled;
 }
 
 // Whether none of NaN voxel k's earlier interior neighbours is NaN (one thread).
@@ -113,12 +114,13 @@ constexpr int kLooks = 256;  // passes over a warp's pending voxels per launch
 __global__ void __launch_bounds__(256) fill_kernel(float *vol, int nx, int ny, int nz, int lo,
                                                    const int *__restrict__ list,
                                                    const int *__restrict__ count,
-                                                   unsigned long long *fills) {
+                                                   unsigned long long *fills,
+                                                   unsigned long long *nan_medians) {
   const int n = *count;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  unsigned filled = 0;
+  unsigned filled = 0, nans = 0;
   for (int look = 0; look < kLooks; ++look) {
     bool left = false;
     // the warp's voxels are w, w + nwarps, ...: 32 of them are tested at once, the pending taken
@@ -136,22 +138,23 @@ __global__ void __launch_bounds__(256) fill_kernel(float *vol, int nx, int ny, i
       while (todo) {
         const int j = __ffs(todo) - 1;
         todo &= todo - 1;
-        if (try_fill(vol, nx, ny, nz, lo, __shfl_sync(0xffffffffu, k, j), lane))
-          ++filled;
-        else
-          left = true;
+        const Look r = try_fill(vol, nx, ny, nz, lo, __shfl_sync(0xffffffffu, k, j), lane);
+        filled += r == kFilled;
+        nans += r == kNanMedian && look == 0;
+        left |= r == kWaits;
       }
       if (base > n - 1 - 32 * nwarps) break;  // (the next base could overflow)
     }
     if (!left) break;
   }
   if (lane == 0 && filled) atomicAdd(fills, (unsigned long long)filled);
+  if (lane == 0 && nans) atomicAdd(nan_medians, (unsigned long long)nans);
 }
 
 }  // namespace
 
 size_t regularize_scratch_bytes(long long nvox) {
-  // An index list of at most nvox entries, its length and a fill counter.
+  // An index list of at most nvox entries, its length and two counters.
   return (size_t)nvox * sizeof(int) + 64;
 }
 
@@ -163,7 +166,7 @@ cudaError_t launch_regularize(float *vol, int nx, int ny, int nz, int nh, void *
   if (nx <= 2 * lo || ny <= 2 * lo || nz <= 2 * lo) return cudaSuccess;
   char *base = static_cast<char *>(scratch);
   struct Counters {
-    unsigned long long fills;
+    unsigned long long fills, nan_medians;
     int listed;
   } host{};
   int *count = reinterpret_cast<int *>(base + offsetof(Counters, listed));
@@ -175,22 +178,32 @@ cudaError_t launch_regularize(float *vol, int nx, int ny, int nz, int nh, void *
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   collect_nan_kernel<<<sms * 8, 256, 0, stream>>>(vol, nx, ny, nz, lo, list, count);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  unsigned long long *fills = reinterpret_cast<unsigned long long *>(base);
+  long long filled = 0;
   int launches = 0;
-  for (unsigned long long before = 0;; before = host.fills) {
+  for (;;) {
+    const Counters before = host;
     // (every CTA resident: a warp may wait for a fill of another)
     fill_kernel<<<sms * 4, 256, 0, stream>>>(vol, nx, ny, nz, lo, list, count,
-                                             reinterpret_cast<unsigned long long *>(base));
+                                             fills, fills + 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(&host, base, sizeof(host), cudaMemcpyDeviceToHost, stream)) !=
         cudaSuccess)
       return e;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
     ++launches;
-    // a launch that filled nothing means only voxels with no non-NaN neighbour remain (possible
-    // only with NaN in the border), and no later one could fill them either
-    if (host.fills >= (unsigned long long)host.listed || host.fills == before) break;
+    // A launch that filled nothing means that only voxels with no non-NaN neighbour remain (possible
+    // only with NaN in the border) and those whose median is NaN, with what waits for either, and no
+    // later one could fill them. A NaN median counts as a fill, as the voxel's one visit in a sweep
+    // does; the volume stood still in this launch, so its first look met each of them once.
+    filled = (long long)host.fills;
+    if (host.fills >= (unsigned long long)host.listed) break;
+    if (host.fills == before.fills) {
+      filled += (long long)(host.nan_medians - before.nan_medians);
+      break;
+    }
   }
-  if (fills_out) *fills_out = (long long)host.fills;
+  if (fills_out) *fills_out = filled;
   if (rounds_out) *rounds_out = launches;
   return cudaSuccess;
 }
