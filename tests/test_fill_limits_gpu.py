@@ -76,3 +76,21 @@ def test_nan_medians_beside_a_chain(chain, boxes):
     ref, fills = fill_rule(vol, 3)
     assert fills == chain + boxes and not np.isnan(ref[2, 2]).any()
     check(vol, 3)
+
+
+@pytest.mark.parametrize("shape,nh", [((112, 222, 222), 7), ((40, 90, 100), 3)])
+def test_what_nothing_can_fill_ends_soon(shape, nh):
+    """All NaN: each launch only looks. Measured 0.77 ms for the larger volume, 0.88 with a launch
+    per round; 76 ms when every look of a launch was taken."""
+    vol = torch.full(shape, float("nan"), device="cuda")
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    times = []
+    with pct.Handle(0) as h:
+        for _ in range(4):
+            a.record()
+            assert h.regularize_device(vol.data_ptr(), shape[1], shape[2], shape[0], nh) == 0
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+    assert bool(vol.isnan().all())
+    assert min(times[1:]) < 8.0, times
