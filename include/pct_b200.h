@@ -98,6 +98,11 @@ int pct_synthesize(pct_handle *h, const float *img, const float *atlas, const fl
  * `stream` (a cudaStream_t; NULL = the CUDA default stream, as everywhere in this header). Only
  * interior voxels of d_out are written; border voxels keep whatever the caller put there. Asynchronous: errors from the
  * launch are returned, errors during execution surface at the next synchronising call.
+ *
+ * Under stream capture the call allocates nothing: it plans with the scratch that the handle has, so
+ * make the same call once before capturing it. The graph holds the addresses of that scratch. It stays
+ * allocated, whatever later calls on the handle need, until pct_destroy: replay the graph before that,
+ * and order its replays with the handle's other calls as those among themselves.
  */
 int pct_synthesize_device(pct_handle *h, const float *d_img, const float *d_atlas,
                           const float *d_atlas_label, float *d_out, int nx, int ny, int nz,

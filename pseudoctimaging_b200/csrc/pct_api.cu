@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <string>
@@ -20,6 +21,7 @@ namespace {
 struct DevBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
+  bool captured = false;  // a caller's CUDA graph may hold the address
 };
 
 }  // namespace
@@ -34,6 +36,7 @@ struct pct_handle {
   DevBuf err;      // device status word written by kernels with bounded waits
   DevBuf partial;  // per-atlas-group partial sums of the fusion kernel
   DevBuf stage;    // contiguous host->device staging before the pitched repack
+  std::vector<DevBuf> retired;  // captured buffers that were outgrown: kept for their graphs' replays
   unsigned long long wait_test_ns = 0;  // one-shot testing hook, see pct_test_wait_timeout
   int tile_set = 0;                     // register-tile set (pct_autotune / pct_set_tile_set)
   DevBuf batch_stage, batch_meta;       // pct_synthesize_batch: pitched stacks, subject table
@@ -109,7 +112,7 @@ DevBuf take_spare(int device, size_t bytes, size_t most) {
 
 // Whether the block was kept (its last use must be over).
 bool leave_spare(int device, const DevBuf &b) {
-  if (!b.ptr || b.bytes > kSpareBlock) return false;
+  if (!b.ptr || b.captured || b.bytes > kSpareBlock) return false;
   std::lock_guard<std::mutex> lock(spare_mutex);
   size_t total = b.bytes;
   for (const SpareBlock &s : spare_blocks) total += s.buf.bytes;
@@ -135,14 +138,22 @@ int ensure_partial(pct_handle *h, size_t bytes) {
   return ensure(h, h->partial, bytes);
 }
 
-// Grow-only device buffer owned by the handle, subject to the handle's memory cap.
+// Grow-only device buffer owned by the handle, subject to the handle's memory cap. One that a caller's
+// graph was captured with stays allocated when it is outgrown, as long as the handle lives.
 int ensure(pct_handle *h, DevBuf &b, size_t bytes) {
   if (b.bytes >= bytes) return PCT_OK;
-  const size_t others = h->allocated - b.bytes;
+  const size_t others = h->allocated - (b.captured ? 0 : b.bytes);
   if (h->mem_limit && others + bytes > h->mem_limit)
     return fail(h, PCT_ERR_OUT_OF_MEMORY,
                 "allocation of " + std::to_string(bytes) + " bytes exceeds the handle's memory limit");
-  if (b.ptr) {
+  if (b.captured) {
+    try {
+      h->retired.push_back(b);
+    } catch (...) {
+      return fail(h, PCT_ERR_OUT_OF_MEMORY, "out of host memory");
+    }
+    b = DevBuf{};
+  } else if (b.ptr) {
     cudaFree(b.ptr);
     h->allocated -= b.bytes;
     b.ptr = nullptr;
@@ -218,6 +229,12 @@ bool is_capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
+// Marks buffers whose addresses a call being captured has put into the caller's graph.
+void note_capture(cudaStream_t s, std::initializer_list<DevBuf *> used) {
+  if (!is_capturing(s)) return;
+  for (DevBuf *b : used) b->captured = b->captured || b->ptr;
+}
+
 // Plans the plain kernel and makes room for its partial sums. The plan keeps to what the handle's
 // memory cap leaves for them once its other buffers have grown by `others_grow` bytes, and to what
 // is there already when the stream is being captured (no allocation then) or the device has no
@@ -233,8 +250,10 @@ int plan_fusion(pct_handle *h, const pct::Geometry &g, size_t others_grow, cudaS
     const size_t others = h->allocated - h->partial.bytes + others_grow;
     limit = h->mem_limit > others ? h->mem_limit - others : 0;
   }
-  if (is_capturing(s)) limit = std::min(limit, h->partial.bytes);
+  const bool capturing = is_capturing(s);
+  if (capturing) limit = std::min(limit, h->partial.bytes);
   PCT_CUDA(h, make(limit));
+  if (capturing && plan->partial_bytes) h->partial.captured = true;
   if (!plan->partial_bytes || !ensure_partial(h, plan->partial_bytes)) return PCT_OK;
   h->last_error.clear();
   PCT_CUDA(h, make(h->partial.bytes));
@@ -310,6 +329,7 @@ int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in
                                             s));
     in = pct::SlabInputs{in.img, static_cast<const float *>(h->atlas.ptr),
                          static_cast<const float *>(h->label.ptr), pitch};
+    note_capture(s, {&h->atlas, &h->label});
   }
   pct::FusePlan plan;
   if ((st = plan_fusion(h, g, 0, s, &plan, &runs))) return st;
@@ -346,6 +366,7 @@ int launch_learned_path(pct_handle *h, const pct::Geometry &g, const pct::SlabIn
       return fail(h, PCT_ERR_UNSUPPORTED, "the centre prior needs at least 4 interior x-rows");
     int st = ensure(h, h->learned, pct::learned::infer_scratch_bytes(g));
     if (st) return st;
+    note_capture(s, {&h->learned});
     bool done = false;
     if ((st = launch_prior_tiles(h, g, in, d_out, div, s, &done))) return st;
     if (!done)
@@ -372,7 +393,9 @@ int launch_learned_path(pct_handle *h, const pct::Geometry &g, const pct::SlabIn
   if (h->learned_conf > 0.f && g.nh == 11) {
     if ((st = ensure(h, h->partial, pct::learned::fallback_partial_bytes(g)))) return st;
     fb_partial = static_cast<float *>(h->partial.ptr);
+    note_capture(s, {&h->partial});
   }
+  note_capture(s, {&h->learned});
   PCT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), s));
   PCT_CUDA(h, pct::learned::launch_learned(g, pct::learned::model_weights(h->model), in, d_out, div,
                                            h->learned_conf, h->learned_block, h->learned_level,
@@ -408,7 +431,9 @@ int launch_tc_path(pct_handle *h, const pct::Geometry &g, const pct::SlabInputs 
                                   cudaMemcpyDeviceToDevice, s));
     tin = pct::SlabInputs{in.img, static_cast<const float *>(h->atlas.ptr),
                           static_cast<const float *>(h->label.ptr), pitch};
+    note_capture(s, {&h->atlas, &h->label});
   }
+  note_capture(s, {&h->tcbuf});
   int *err = static_cast<int *>(h->err.ptr);
   PCT_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), s));
   PCT_CUDA(h, pct::tc::launch_tc(g, tin, d_out, div, bf16, err, dbg_top, h->tcbuf.ptr, s));
@@ -888,11 +913,12 @@ int pct_destroy(pct_handle *h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   // (the partial sums are left to the next handle once nothing can use them any more)
-  if (h->partial.ptr && cudaDeviceSynchronize() == cudaSuccess && leave_spare(h->device, h->partial))
+  if (h->partial.ptr && !h->partial.captured && cudaDeviceSynchronize() == cudaSuccess && leave_spare(h->device, h->partial))
     h->partial = DevBuf{};
   for (DevBuf *b : {&h->img, &h->atlas, &h->label, &h->out, &h->scratch, &h->err, &h->partial,
                     &h->stage, &h->batch_stage, &h->batch_meta, &h->learned, &h->tcbuf})
     if (b->ptr) cudaFree(b->ptr);
+  for (const DevBuf &b : h->retired) cudaFree(b.ptr);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   if (h->compute_stream) cudaStreamDestroy(h->compute_stream);
   if (h->output_stream) cudaStreamDestroy(h->output_stream);
@@ -1061,6 +1087,7 @@ int pct_synthesize_device(pct_handle *h, const float *d_img, const float *d_atla
                                             g.ny, pitch, s));
     in = pct::SlabInputs{d_img, static_cast<const float *>(h->atlas.ptr),
                          static_cast<const float *>(h->label.ptr), pitch};
+    note_capture(s, {&h->atlas, &h->label});
   }
   return launch_path(h, g, in, d_out, div, exec_choice, s);
 }
