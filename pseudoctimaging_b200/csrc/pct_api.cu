@@ -912,10 +912,13 @@ int pct_destroy(pct_handle *h) {
   if (!h) return PCT_ERR_INVALID_ARG;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  // (the partial sums are left to the next handle once nothing can use them any more)
-  if (h->partial.ptr && !h->partial.captured && cudaDeviceSynchronize() == cudaSuccess && leave_spare(h->device, h->partial))
-    h->partial = DevBuf{};
-  for (DevBuf *b : {&h->img, &h->atlas, &h->label, &h->out, &h->scratch, &h->err, &h->partial,
+  // The partial sums are left to the next handle once nothing can use them any more: cudaFree waits
+  // for the work of all streams, and whatever used them has a status word. (cudaDeviceSynchronize
+  // would do as well, but it breaks a capture that is under way on any other stream.)
+  const bool idle = h->err.ptr && cudaFree(h->err.ptr) == cudaSuccess;
+  h->err = DevBuf{};
+  if (idle && leave_spare(h->device, h->partial)) h->partial = DevBuf{};
+  for (DevBuf *b : {&h->img, &h->atlas, &h->label, &h->out, &h->scratch, &h->partial,
                     &h->stage, &h->batch_stage, &h->batch_meta, &h->learned, &h->tcbuf})
     if (b->ptr) cudaFree(b->ptr);
   for (const DevBuf &b : h->retired) cudaFree(b.ptr);

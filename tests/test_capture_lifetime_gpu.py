@@ -68,3 +68,52 @@ def test_replay_after_larger_calls(small, choice):
         torch.cuda.synchronize()
         np.testing.assert_array_equal(big[3].cpu().numpy(), first.cpu().numpy())
         other.close()
+
+
+@pytest.mark.parametrize("mode", ["relaxed", "thread_local"])
+def test_closing_a_handle_leaves_captures_alone(mode):
+    """A handle with partial sums is closed (in another thread) while a stream is being captured."""
+    import threading
+
+    h = pct.Handle(0)
+    d = volumes(64, 64, 32, 1, 5)
+    call(h, d, pct.EXEC_B200_FP32)
+    torch.cuda.synchronize()
+    with pct.Handle(0):  # not the last handle: its partial sums are kept
+        x = torch.zeros(16, device="cuda")
+        g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            g.capture_begin(capture_error_mode=mode)
+            x.add_(1)
+            t = threading.Thread(target=h.close)
+            t.start()
+            t.join()
+            x.add_(1)
+            g.capture_end()
+        g.replay()
+        torch.cuda.synchronize()
+        assert float(x[0]) == 2.0
+
+
+def test_sums_are_passed_on_only_when_idle():
+    """A handle closed right after an asynchronous call: the next handle's call, which takes over the
+    partial sums, waits for it."""
+    d, e = volumes(64, 64, 32, 3, 6), volumes(64, 64, 32, 3, 7)
+    assert 0 < pct.query_plan(64, 64, 32, 3, NH)["scratch_bytes"] <= 32 << 20
+    refs = []
+    for v in (d, e):
+        with pct.Handle(0) as h:
+            call(h, v, pct.EXEC_B200_FP32)
+            torch.cuda.synchronize()
+        refs.append(v[3].clone())
+        v[3].zero_()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    with pct.Handle(0):
+        for _ in range(10):
+            for v, s in zip((d, e), streams):
+                with torch.cuda.stream(s), pct.Handle(0) as h:
+                    call(h, v, pct.EXEC_B200_FP32)
+    torch.cuda.synchronize()
+    for v, ref in zip((d, e), refs):
+        np.testing.assert_array_equal(v[3].cpu().numpy(), ref.cpu().numpy())
