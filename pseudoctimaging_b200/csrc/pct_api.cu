@@ -127,12 +127,10 @@ bool leave_spare(int device, const DevBuf &b) {
 
 int ensure(pct_handle *h, DevBuf &b, size_t bytes);
 
-// ensure for the partial sums: from the spare blocks first.
-int ensure_partial(pct_handle *h, size_t bytes) {
+// ensure for the partial sums, within `limit` bytes: from the spare blocks first.
+int ensure_partial(pct_handle *h, size_t bytes, size_t limit) {
   if (!h->partial.ptr && bytes <= kSpareBlock) {
-    const size_t room = h->mem_limit ? (h->mem_limit > h->allocated ? h->mem_limit - h->allocated : 0)
-                                     : kSpareBlock;
-    h->partial = take_spare(h->device, bytes, std::min(room, 4 * bytes));
+    h->partial = take_spare(h->device, bytes, std::min(limit, 4 * bytes));
     h->allocated += h->partial.bytes;
   }
   return ensure(h, h->partial, bytes);
@@ -254,7 +252,7 @@ int plan_fusion(pct_handle *h, const pct::Geometry &g, size_t others_grow, cudaS
   if (capturing) limit = std::min(limit, h->partial.bytes);
   PCT_CUDA(h, make(limit));
   if (capturing && plan->partial_bytes) h->partial.captured = true;
-  if (!plan->partial_bytes || !ensure_partial(h, plan->partial_bytes)) return PCT_OK;
+  if (!plan->partial_bytes || !ensure_partial(h, plan->partial_bytes, limit)) return PCT_OK;
   h->last_error.clear();
   PCT_CUDA(h, make(h->partial.bytes));
   return PCT_OK;
