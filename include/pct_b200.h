@@ -76,7 +76,8 @@ int pct_destroy(pct_handle *h);
  * handle's own stream. The calls still synchronise on it before returning. */
 int pct_set_stream(pct_handle *h, void *stream);
 /* Cap on the bytes the handle may allocate (0 = unlimited). Exceeding it returns
- * PCT_ERR_OUT_OF_MEMORY without calling the allocator. */
+ * PCT_ERR_OUT_OF_MEMORY without an allocation. Scratch that only makes a call faster (partial sums,
+ * staged or repacked stacks) is kept between calls, but gives way to what a later call needs. */
 int pct_set_memory_limit(pct_handle *h, size_t bytes);
 
 /*

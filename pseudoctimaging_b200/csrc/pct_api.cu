@@ -22,6 +22,7 @@ struct DevBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
   bool captured = false;  // a caller's CUDA graph may hold the address
+  unsigned call = 0;      // the handle's last call that used it
 };
 
 }  // namespace
@@ -32,6 +33,7 @@ struct pct_handle {
   cudaStream_t user_stream = nullptr;  // set by pct_set_stream for host-pointer calls
   size_t mem_limit = 0;  // 0 = unlimited
   size_t allocated = 0;
+  unsigned call = 0;  // counts the entry points' calls (DevBuf::call)
   DevBuf img, atlas, label, out, scratch;
   DevBuf err;      // device status word written by kernels with bounded waits
   DevBuf partial;  // per-atlas-group partial sums of the fusion kernel
@@ -110,6 +112,19 @@ DevBuf take_spare(int device, size_t bytes, size_t most) {
   return b;
 }
 
+// Frees the device's spare blocks; whether there were any.
+bool free_spares(int device) {
+  std::lock_guard<std::mutex> lock(spare_mutex);
+  bool any = false;
+  for (size_t i = spare_blocks.size(); i-- > 0;) {
+    if (spare_blocks[i].device != device) continue;
+    cudaFree(spare_blocks[i].buf.ptr);
+    spare_blocks.erase(spare_blocks.begin() + i);
+    any = true;
+  }
+  return any;
+}
+
 // Whether the block was kept (its last use must be over).
 bool leave_spare(int device, const DevBuf &b) {
   if (!b.ptr || b.captured || b.bytes > kSpareBlock) return false;
@@ -125,21 +140,16 @@ bool leave_spare(int device, const DevBuf &b) {
   return true;
 }
 
-int ensure(pct_handle *h, DevBuf &b, size_t bytes);
-
-// ensure for the partial sums, within `limit` bytes: from the spare blocks first.
-int ensure_partial(pct_handle *h, size_t bytes, size_t limit) {
-  if (!h->partial.ptr && bytes <= kSpareBlock) {
-    h->partial = take_spare(h->device, bytes, std::min(limit, 4 * bytes));
-    h->allocated += h->partial.bytes;
-  }
-  return ensure(h, h->partial, bytes);
+// Frees one of the handle's buffers (cudaFree waits for the work that uses it).
+void release(pct_handle *h, DevBuf &b) {
+  if (b.ptr) cudaFree(b.ptr);
+  h->allocated -= b.bytes;
+  b = DevBuf{};
 }
 
-// Grow-only device buffer owned by the handle, subject to the handle's memory cap. One that a caller's
-// graph was captured with stays allocated when it is outgrown, as long as the handle lives.
-int ensure(pct_handle *h, DevBuf &b, size_t bytes) {
-  if (b.bytes >= bytes) return PCT_OK;
+// Grows b to `bytes` or more, subject to the handle's memory cap. A buffer that a caller's graph was
+// captured with stays allocated when it is outgrown, as long as the handle lives.
+int grow(pct_handle *h, DevBuf &b, size_t bytes) {
   const size_t others = h->allocated - (b.captured ? 0 : b.bytes);
   if (h->mem_limit && others + bytes > h->mem_limit)
     return fail(h, PCT_ERR_OUT_OF_MEMORY,
@@ -151,12 +161,8 @@ int ensure(pct_handle *h, DevBuf &b, size_t bytes) {
       return fail(h, PCT_ERR_OUT_OF_MEMORY, "out of host memory");
     }
     b = DevBuf{};
-  } else if (b.ptr) {
-    cudaFree(b.ptr);
-    h->allocated -= b.bytes;
-    b.ptr = nullptr;
-    b.bytes = 0;
   }
+  release(h, b);
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) {
@@ -167,6 +173,57 @@ int ensure(pct_handle *h, DevBuf &b, size_t bytes) {
   b.bytes = bytes;
   h->allocated += bytes;
   return PCT_OK;
+}
+
+// A buffer that the call can do without (partial sums, stacks copied for a faster path): nothing gives
+// way to it.
+int try_ensure(pct_handle *h, DevBuf &b, size_t bytes) {
+  const int st = b.bytes >= bytes ? PCT_OK : grow(h, b, bytes);
+  if (!st) b.call = h->call;
+  return st;
+}
+
+// A buffer that the call needs. Where the handle's cap or the device leaves no room for it, partial
+// sums and copied stacks that this call does not use give way, one by one, and then the partial sums
+// of closed handles.
+int ensure(pct_handle *h, DevBuf &b, size_t bytes) {
+  int st = try_ensure(h, b, bytes);
+  if (st == PCT_ERR_OUT_OF_MEMORY) {
+    b.call = h->call;  // (no candidate itself)
+    DevBuf *const candidates[] = {&h->partial, &h->stage, &h->atlas, &h->label};
+    auto gives_way = [&](const DevBuf *o) { return o->ptr && !o->captured && o->call != h->call; };
+    size_t stays = h->allocated - (b.captured ? 0 : b.bytes);
+    for (const DevBuf *o : candidates)
+      if (gives_way(o)) stays -= o->bytes;
+    if (h->mem_limit && stays + bytes > h->mem_limit) return st;
+    for (DevBuf *o : candidates) {
+      if (st != PCT_ERR_OUT_OF_MEMORY || !gives_way(o)) continue;
+      release(h, *o);
+      st = try_ensure(h, b, bytes);
+    }
+    if (st == PCT_ERR_OUT_OF_MEMORY && free_spares(h->device)) st = try_ensure(h, b, bytes);
+    if (!st) h->last_error.clear();
+  }
+  return st;
+}
+
+// try_ensure for the partial sums, within `limit` bytes: from the spare blocks first.
+int ensure_partial(pct_handle *h, size_t bytes, size_t limit) {
+  if (!h->partial.ptr && bytes <= kSpareBlock) {
+    h->partial = take_spare(h->device, bytes, std::min(limit, 4 * bytes));
+    h->allocated += h->partial.bytes;
+  }
+  return try_ensure(h, h->partial, bytes);
+}
+
+// What the cap leaves for optional buffer b once the others have grown by `others_grow` bytes. One that
+// is larger already would take room from them, so it goes.
+size_t room_for(pct_handle *h, DevBuf &b, size_t others_grow) {
+  if (!h->mem_limit) return SIZE_MAX;
+  const size_t others = h->allocated - (b.captured ? 0 : b.bytes) + others_grow;
+  const size_t room = h->mem_limit > others ? h->mem_limit - others : 0;
+  if (b.bytes > room && !b.captured) release(h, b);
+  return room;
 }
 
 int check_choice(pct_handle *h, int exec_choice) {
@@ -210,7 +267,9 @@ int check_shape(pct_handle *h, int nx, int ny, int nz, int num, int nh, double d
   return PCT_OK;
 }
 
+// Begins a call: what it allocates from here on is in use until the next one.
 int select_device(pct_handle *h) {
+  ++h->call;
   PCT_CUDA(h, cudaSetDevice(h->device));
   return PCT_OK;
 }
@@ -235,26 +294,25 @@ void note_capture(cudaStream_t s, std::initializer_list<DevBuf *> used) {
 
 // Plans the plain kernel and makes room for its partial sums. The plan keeps to what the handle's
 // memory cap leaves for them once its other buffers have grown by `others_grow` bytes, and to what
-// is there already when the stream is being captured (no allocation then) or the device has no
-// more: one group needs none, so a plan always exists.
+// is there already when the stream is being captured (no allocation then; none at all under a cap,
+// where a buffer that a graph holds could not give way) or the device has no more: one group needs
+// none, so a plan always exists.
 int plan_fusion(pct_handle *h, const pct::Geometry &g, size_t others_grow, cudaStream_t s,
                 pct::FusePlan *plan, const pct::OffsetRuns *runs = nullptr) {
   auto make = [&](size_t limit) {
     return runs ? pct::fuse_runs_plan(g, *runs, limit, plan)
                 : pct::fuse_tma_plan(g, h->tile_set, limit, plan);
   };
-  size_t limit = SIZE_MAX;
-  if (h->mem_limit) {
-    const size_t others = h->allocated - h->partial.bytes + others_grow;
-    limit = h->mem_limit > others ? h->mem_limit - others : 0;
-  }
   const bool capturing = is_capturing(s);
-  if (capturing) limit = std::min(limit, h->partial.bytes);
+  const size_t limit = !capturing ? room_for(h, h->partial, others_grow)
+                                  : h->mem_limit ? 0 : h->partial.bytes;
   PCT_CUDA(h, make(limit));
+  if (plan->partial_bytes && ensure_partial(h, plan->partial_bytes, limit)) {
+    h->last_error.clear();
+    PCT_CUDA(h, make(std::min(limit, h->partial.bytes)));
+    h->partial.call = h->call;
+  }
   if (capturing && plan->partial_bytes) h->partial.captured = true;
-  if (!plan->partial_bytes || !ensure_partial(h, plan->partial_bytes, limit)) return PCT_OK;
-  h->last_error.clear();
-  PCT_CUDA(h, make(h->partial.bytes));
   return PCT_OK;
 }
 
@@ -317,8 +375,10 @@ int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in
     const long long rows = (long long)g.num * g.nz * g.nx;
     const size_t bytes = (size_t)rows * pitch * sizeof(float);
     const bool there = h->atlas.bytes >= bytes && h->label.bytes >= bytes;
-    if (in.pitch != g.ny || (!there && is_capturing(s))) return PCT_OK;
-    if (ensure(h, h->atlas, bytes) || ensure(h, h->label, bytes)) {
+    if (in.pitch != g.ny || (is_capturing(s) && (!there || h->mem_limit))) return PCT_OK;
+    const bool grown = h->atlas.bytes < bytes;
+    if (try_ensure(h, h->atlas, bytes) || try_ensure(h, h->label, bytes)) {
+      if (grown && !h->atlas.captured) release(h, h->atlas);  // (the rescoring reads neither)
       h->last_error.clear();
       return PCT_OK;
     }
@@ -573,12 +633,11 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
                            (pitch != g.ny ? grow(h->stage, rows * g.ny * sizeof(float)) : 0),
                        s, &pl);
   if (st) return st;
-  if (pl.atlas_groups < 2 || h->wait_test_ns) return PCT_ERR_UNSUPPORTED;
-  if ((st = ensure(h, h->atlas, rows * pitch * sizeof(float))) ||
-      (st = ensure(h, h->label, rows * pitch * sizeof(float))) || (st = ensure(h, h->err, 16)))
-    return st;
-  if (pitch != g.ny && ensure(h, h->stage, 2 * rows * g.ny * sizeof(float))) {
-    h->last_error.clear();  // over the handle's memory cap: the one-upload path needs half
+  if (pl.atlas_groups < 2 || h->wait_test_ns || ensure(h, h->atlas, rows * pitch * sizeof(float)) ||
+      ensure(h, h->label, rows * pitch * sizeof(float)) || ensure(h, h->err, 16) ||
+      (pitch != g.ny && try_ensure(h, h->stage, 2 * rows * g.ny * sizeof(float)))) {
+    // (no room: the one-upload path needs half the staging, and takes the partial sums' place)
+    h->partial.call = 0;
     return PCT_ERR_UNSUPPORTED;
   }
   struct Part {
@@ -1441,17 +1500,12 @@ int stage_batch(pct_handle *h, const pct_subject *subs, int n, const std::vector
   return PCT_OK;
 }
 
-// Plans a batch's atlas groups within what the handle's memory cap leaves for `buf` and makes room
-// for their partial sums; without it every subject is one group, which needs none.
+// Plans a batch's atlas groups and makes room for their partial sums in `buf`, at most `limit` bytes;
+// without it every subject is one group, which needs none.
 int plan_batch(pct_handle *h, const std::vector<pct::Geometry> &geo, int set, DevBuf &buf,
-               pct::BatchPlan *plan) {
-  size_t limit = SIZE_MAX;
-  if (h->mem_limit) {
-    const size_t others = h->allocated - buf.bytes;
-    limit = h->mem_limit > others ? h->mem_limit - others : 0;
-  }
+               size_t limit, pct::BatchPlan *plan) {
   PCT_CUDA(h, pct::plan_batch(geo.data(), (int)geo.size(), set, limit, plan));
-  if (!plan->partial_bytes || !ensure(h, buf, plan->partial_bytes)) return PCT_OK;
+  if (!plan->partial_bytes || !try_ensure(h, buf, plan->partial_bytes)) return PCT_OK;
   h->last_error.clear();
   PCT_CUDA(h, pct::plan_batch(geo.data(), (int)geo.size(), set, 0, plan));
   return PCT_OK;
@@ -1469,7 +1523,7 @@ int run_batch_once(pct_handle *h, const pct_subject *subs, int n, int set, cudaS
   std::vector<pct::BatchSubjectIn> in;
   if ((st = stage_batch(h, subs, n, geo, h->batch_stage.ptr, in, s))) return st;
   pct::BatchPlan plan;
-  if ((st = plan_batch(h, geo, set, h->partial, &plan))) return st;
+  if ((st = plan_batch(h, geo, set, h->partial, room_for(h, h->partial, 0), &plan))) return st;
   int *err = static_cast<int *>(h->err.ptr);
   PCT_CUDA(h, cudaMemsetAsync(err, 0, 2 * sizeof(int), s));
   pct::BatchSetup setup;
@@ -1577,7 +1631,9 @@ int pct_batch_create(pct_handle *h, const pct_subject *subjects, int n, void *st
       (st = ensure(h, b->meta, pct::batch_scratch_bytes(n))) || (st = ensure(h, b->err, 16)))
     return cleanup(st);
   pct::BatchPlan plan;
-  if ((st = plan_batch(h, geo, h->tile_set, b->partial, &plan))) return cleanup(st);
+  // (under a cap none: the batch would hold it as long as it lives, and no later call could have it)
+  if ((st = plan_batch(h, geo, h->tile_set, b->partial, h->mem_limit ? 0 : SIZE_MAX, &plan)))
+    return cleanup(st);
   b->bytes = b->stage.bytes + b->meta.bytes + b->err.bytes + b->partial.bytes;
   std::vector<pct::BatchSubjectIn> in;
   pct::BatchSetup setup;
