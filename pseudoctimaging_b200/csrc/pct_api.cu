@@ -551,9 +551,9 @@ cudaError_t download(pct_handle *h, void *dst, const void *src, size_t bytes, cu
 
 // Begins staging the three uploads of the one-upload path.
 void begin_uploads(pct_handle *h, const pct::Geometry &g, const float *img, const float *atlas,
-                   const float *label) {
+                   const float *label, cudaStream_t s) {
   const size_t vol = (size_t)g.nvox() * sizeof(float);
-  h->stager.begin(h->device, {{img, vol}, {atlas, vol * g.num}, {label, vol * g.num}});
+  h->stager.begin(h->device, {{img, vol}, {atlas, vol * g.num}, {label, vol * g.num}}, s);
 }
 
 // Copies host atlas volumes [num*nz*nx][ny] into a pitched device stack for TMA: one
@@ -778,7 +778,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
         jobs.push_back({stack + ((size_t)a * g.nz + p.z0) * plane, whole ? bytes * (p.a1 - p.a0) : bytes});
   }
   StageScope staging{h->stager};
-  h->stager.begin(h->device, jobs);
+  h->stager.begin(h->device, jobs, s);
   st = PCT_OK;
   for (size_t k = 0; k < parts.size() && !st; ++k) st = run_part(k);
   h->stager.end();
@@ -1182,7 +1182,7 @@ int pct_synthesize(pct_handle *h, const float *img, const float *atlas, const fl
     h->last_error.clear();
   }
   StageScope staging{h->stager};
-  begin_uploads(h, g, img, atlas, atlas_label);
+  begin_uploads(h, g, img, atlas, atlas_label, s);
   PCT_CUDA(h, upload(h, h->img.ptr, img, vol, s));
   if ((st = stage_pitched_h2d(h, h->atlas, atlas, g, s)) ||
       (st = stage_pitched_h2d(h, h->label, atlas_label, g, s)))
@@ -1331,7 +1331,7 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
   if (st == PCT_ERR_UNSUPPORTED) {  // one upload, then the path
     h->last_error.clear();
     StageScope staging{h->stager};
-    begin_uploads(h, g, img, atlas_mri, atlas_ct_hu);
+    begin_uploads(h, g, img, atlas_mri, atlas_ct_hu, s);
     PCT_CUDA(h, upload(h, d_img, img, vol, s));
     if ((st = stage_pitched_h2d(h, h->atlas, atlas_mri, g, s)) ||
         (st = stage_pitched_h2d(h, h->label, atlas_ct_hu, g, s)))

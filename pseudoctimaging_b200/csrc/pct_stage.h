@@ -33,10 +33,11 @@ class HostStager {
   // Whether p is plain pageable memory (pinned, managed and device memory are copied directly).
   static bool pageable(const void *p);
 
-  // Starts staging `jobs` in order. False (nothing started, the caller copies directly) when they are
-  // too small to gain, no slots are at hand and too little was copied yet to pin some, or the slots
-  // or threads cannot be had.
-  bool begin(int device, const std::vector<Job> &jobs);
+  // Starts staging `jobs` in order, once the work that `s` (the stream of the transfers, or the one
+  // they follow) already has is done. False (nothing started, the caller copies directly) when they
+  // are too small to gain, no slots are at hand and too little was copied yet to pin some, or the
+  // slots or threads cannot be had.
+  bool begin(int device, const std::vector<Job> &jobs, cudaStream_t s);
   bool active() const { return !threads_.empty(); }
   // The next job's transfer, enqueued on s. Jobs must be taken in the order given to begin.
   cudaError_t copy(void *dst, const void *src, size_t bytes, cudaStream_t s);
@@ -46,8 +47,8 @@ class HostStager {
 
   // Whether a download of this size to p is worth staging.
   static bool takes(const void *p, size_t bytes) { return bytes >= kMinBytes && pageable(p); }
-  // Device to pageable host memory, complete on return. Falls back to one direct copy (and waits
-  // for it) where the slots or threads cannot be had.
+  // Device to pageable host memory, complete on return; waits for the work that s already has first.
+  // Falls back to one direct copy (and waits for it) where the slots or threads cannot be had.
   cudaError_t download(int device, void *dst, const void *src, size_t bytes, cudaStream_t s);
 
   static constexpr int kSlots = 8;
