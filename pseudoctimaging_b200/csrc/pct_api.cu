@@ -536,6 +536,12 @@ struct StageScope {
   ~StageScope() { stager.end(); }
 };
 
+// Ends a host-pointer call on every way out of it.
+struct HostCallScope {
+  pct::HostStager &stager;
+  ~HostCallScope() { stager.pin_ahead(); }
+};
+
 // One upload of a host-pointer call, through the handle's staging when the call began it.
 cudaError_t upload(pct_handle *h, void *dst, const void *src, size_t bytes, cudaStream_t s) {
   if (h->stager.active()) return h->stager.copy(dst, src, bytes, s);
@@ -1166,6 +1172,7 @@ int pct_synthesize(pct_handle *h, const float *img, const float *atlas, const fl
   if (st) return st;
   st = select_device(h);
   if (st) return st;
+  HostCallScope call{h->stager};
   const size_t vol = (size_t)g.nvox() * sizeof(float);
   if ((st = ensure(h, h->img, vol)) || (st = ensure(h, h->out, vol))) return st;
   cudaStream_t s = h->user_stream ? h->user_stream : h->stream;
@@ -1316,6 +1323,7 @@ int pct_run_pipeline(pct_handle *h, const float *img, const float *atlas_mri,
   if (st) return st;
   st = select_device(h);
   if (st) return st;
+  HostCallScope call{h->stager};
   const size_t vol = (size_t)g.nvox() * sizeof(float);
   if ((st = ensure(h, h->img, vol)) || (st = ensure(h, h->out, vol))) return st;
   if (regularize && (st = ensure(h, h->scratch, pct::regularize_scratch_bytes(g.nvox())))) return st;

@@ -47,6 +47,9 @@ class HostStager {
 
   // Whether a download of this size to p is worth staging.
   static bool takes(const void *p, size_t bytes) { return bytes >= kMinBytes && pageable(p); }
+  // Ends a call: has slots pinned for later ones if it asked for them.
+  void pin_ahead();
+
   // Device to pageable host memory, complete on return; waits for the work that s already has first.
   // Falls back to one direct copy (and waits for it) where the slots or threads cannot be had.
   cudaError_t download(int device, void *dst, const void *src, size_t bytes, cudaStream_t s);
@@ -54,10 +57,19 @@ class HostStager {
   static constexpr int kSlots = 8;
   static constexpr size_t kSlotBytes = 2u << 20;
   static constexpr size_t kMinBytes = 12u << 20;  // below, thread start and hand-over eat the gain
-  // A stager without slots copies directly until it has been asked for this much: pinning slots takes
-  // 2.6 ms and staging gains 0.04 to 0.065 ms per MB, so a handle that makes one small call pays
-  // nothing for slots and one that stays pays at most about as much again as they cost.
-  static constexpr size_t kPinBytes = 60u << 20;
+  // A stager without slots copies directly until it has been asked for kPinBytes: pinning slots takes
+  // 2.6 ms and staging gains 0.04 to 0.065 ms per MB. From then on a call of kPinCall or more, which
+  // gains about what they cost, pins them itself. After a smaller call a thread of its own does, for
+  // later calls, which copy directly until it has. (20 MB calls take 1.4 ms; one that pinned in its own
+  // time took 3.1. Now a call that comes while the thread pins takes 2.3, for the driver's lock, and one
+  // that comes 5 ms later 1.4.)
+  static constexpr size_t kPinBytes = 60u << 20, kPinCall = 48u << 20;
+
+  struct Block {  // pinned slots and the events of their transfers
+    int device;
+    char *slots;
+    cudaEvent_t ev[kSlots];
+  };
 
  private:
   struct Chunk {
@@ -70,6 +82,7 @@ class HostStager {
   // ms for 16 MB, where cudaHostAlloc takes 8 to 20 (a new handle's first call on 21 MB of arrays
   // took 17 ms with it, 4.9 with direct copies as now).
   bool reserve(int device, size_t bytes);
+  bool take(const Block &b);
   void release();
   bool start(int device, bool uploads);
   void work(int device, bool uploads);
@@ -78,6 +91,10 @@ class HostStager {
   int device_ = -1;
   char *slots_ = nullptr;
   size_t asked_ = 0;  // bytes that would have been staged while there were no slots
+  int pin_device_ = -1;  // pin_ahead pins slots for it
+  std::thread pinner_;   // makes pinning_, then sets pinned_
+  Block pinning_{};
+  std::atomic<bool> pinned_{false};
   cudaEvent_t ev_[kSlots] = {};
   bool used_[kSlots] = {};  // a transfer was recorded on ev_[k]
 

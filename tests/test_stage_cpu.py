@@ -99,7 +99,7 @@ static bool upload(pct::HostStager &st, const std::vector<char> &v) {
 }
 """
 
-BEGIN = "#define BEGIN(st, v) (st).begin(0, {{(v).data(), (v).size()}}, nullptr)\n"
+BEGIN = "#define BEGIN(st, v) (st).begin(0, {{(v).data(), (v).size()}}, nullptr)\n#define END(st) (st).pin_ahead()\n"
 
 
 def run(tmp_path, main):
@@ -136,3 +136,47 @@ int main() {
 }""")
     assert ok == 1 and queries == 0
     assert cpu < 250, f"{cpu} ms of CPU time for 600 ms of waiting"
+
+
+def test_no_small_call_pays_for_pinning(tmp_path):
+    """Pinning takes 400 ms here. Calls of 25 MB never wait for it, whether they cross the line after which
+    slots are worth having or come while they are pinned; once they are, calls use them. A call that
+    is worth slots by itself pins them at once."""
+    slowest, by_caller, staged, again, handed, at_once, leftover = run(tmp_path, r"""
+int main() {
+  caller = std::this_thread::get_id();
+  register_ms = 400;
+  const std::vector<char> v = data(25u << 20, 1), big = data(62u << 20, 2);
+  double slowest = 0;
+  int staged = 0, again = 0, handed = 0, at_once = 0;
+  {
+    pct::HostStager st;
+    for (int k = 0; k < 6; ++k) {
+      const auto t = Clock::now();
+      if (BEGIN(st, v)) return 4;  // not pinned yet: copied directly
+      END(st);
+      if (ms(t) > slowest) slowest = ms(t);
+    }
+    for (int k = 0; k < 100 && !registered; ++k) std::this_thread::sleep_for(std::chrono::milliseconds(20));
+    std::this_thread::sleep_for(std::chrono::milliseconds(50));
+    staged = upload(st, v);
+    again = upload(st, v);
+    pct::HostStager other;
+    {
+      pct::HostStager closing;
+      for (int k = 0; k < 3; ++k) {
+        BEGIN(closing, v);
+        END(closing);
+      }
+    }  // closed while it pins: the slots pass on
+    handed = upload(other, v);
+  }
+  const bool small_by_caller = registered_by_caller;
+  pct::HostStager st;
+  at_once = upload(st, big);
+  printf("%.1f %d %d %d %d %d %ld\n", slowest, small_by_caller, staged, again, handed, at_once,
+         registered.load());
+}""")
+    assert slowest < 200 and by_caller == 0
+    assert staged == again == handed == at_once == 1
+    assert leftover == 3  # one per stager that asked for slots and found none
