@@ -29,12 +29,15 @@ INCLUDE = REPO / "include"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 HOST_CXX = shutil.which("g++", path="/usr/bin") or "g++"
 COMMON = ["-O3", "-std=c++17", "-lineinfo", f"-ccbin={HOST_CXX}", "-Xcompiler", "-fPIC",
-          f"-I{INCLUDE}", f"-I{CSRC}", f"-I{OBJ}"]
+          "-Xfatbin=-compress-all", f"-I{INCLUDE}", f"-I{CSRC}", f"-I{OBJ}"]
 # Sources that make up the shared library; the CLI main is linked separately against it.
-LIB_SOURCES = ["pct_api.cu", "pct_fuse_tma.cu", "pct_pointwise.cu", "pct_regularize.cu",
-               "pct_noalloc.cu", "pct_synth.cpp", "pct_io.cpp", "pct_learned_train.cu",
+LIB_SOURCES = ["pct_api.cu", "pct_fuse_tma.cu", "pct_fuse_list.cu", "pct_pointwise.cu",
+               "pct_regularize.cu", "pct_noalloc.cu", "pct_synth.cpp", "pct_io.cpp", "pct_learned_train.cu",
                "pct_learned_api.cu", "pct_learned_infer.cu", "pct_tc_fuse.cu", "pct_jit.cpp",
                "pct_mat.cpp", "pct_stage.cpp"]
+# Sources compiled once per value of a macro, each to an object of its own: the driver loads an object's
+# device code as a whole, at the first launch from it.
+VARIANTS = {"pct_fuse_set.cu": ("PCT_TILE_SET", range(8)), "pct_fuse_batch.cu": ("PCT_TILE_SET", range(5))}
 # Device sources that are also compiled at run time (NVRTC): each is embedded as a string in
 # _build/<stem>_src.inc, which the library sources include.
 EMBEDDED = ["pct_rescore.cuh"]
@@ -83,11 +86,14 @@ def _run(cmd: list[str], verbose: bool) -> str:
     return res.stdout + res.stderr
 
 
-def _compile(src: pathlib.Path, force: bool, verbose: bool, ptxas_info: bool) -> tuple[pathlib.Path, str]:
-    obj = OBJ / (src.name + ".o")
+def _compile(src: pathlib.Path, force: bool, verbose: bool, ptxas_info: bool,
+             define: tuple[str, int] | None = None) -> tuple[pathlib.Path, str]:
+    obj = OBJ / (src.name + (f".{define[1]}.o" if define else ".o"))
     if not force and not _stale(obj, [src] + _headers()):
         return obj, ""
     cmd = [nvcc(), *ARCH, *COMMON, "-c", str(src), "-o", str(obj)]
+    if define:
+        cmd.append(f"-D{define[0]}={define[1]}")
     if src.suffix == ".cu" and ptxas_info:
         cmd += ["-Xptxas", "-v"]
     return obj, _run(cmd, verbose)
@@ -100,9 +106,10 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     CLI.parent.mkdir(parents=True, exist_ok=True)
     for name in EMBEDDED:
         _embed(name)
-    srcs = [CSRC / s for s in LIB_SOURCES]
+    jobs = [(CSRC / name, (macro, k)) for name, (macro, ks) in VARIANTS.items() for k in ks]
+    jobs += [(CSRC / name, None) for name in LIB_SOURCES]
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        results = list(ex.map(lambda s: _compile(s, force, verbose, ptxas_info), srcs))
+        results = list(ex.map(lambda j: _compile(j[0], force, verbose, ptxas_info, j[1]), jobs))
     objs = [o for o, _ in results]
     if ptxas_info:
         for _, log in results:

@@ -123,7 +123,7 @@ struct BatchSubjectIn {
 };
 struct BatchSetup {
   bool params_ready = false;
-  int items = 0, blocks = 0, smem = 0, set = 0;
+  int items = 0, blocks = 0, set = 0;
   void *bp_subjects = nullptr;
   int bp_nsub = 0;
   int *bp_err = nullptr;  // status word, then the counter of items taken (both zero at launch)
