@@ -349,7 +349,7 @@ int pct_regularize_device(pct_handle *h, float *d_vol, int nx, int ny, int nz, i
  * while running (for example applications whose device memory belongs to their own pool
  * allocator, or latency-critical loops that forbid allocation after start-up). No counterpart in
  * the reference. Same result as pct_regularize_device; needs no handle and calls no allocator:
- * its scratch is a fixed 64 MiB array inside the library, held by every GPU that loads the
+ * its scratch is a fixed 32 MiB array inside the library, held by every GPU that loads the
  * library until the process exits. Volumes of more than 2^23 voxels (8,388,608) are rejected
  * with PCT_ERR_TOO_LARGE. Runs on the current device. CUDA loads the library's device code
  * lazily, so the array is reserved on a device by the first call of this entry point (or of any

@@ -27,9 +27,9 @@
 namespace {
 
 // Largest volume this entry point accepts, and the scratch it needs: a 64-byte header of
-// counters plus kMaxVoxels index entries, twice over (64 MiB in total, as documented to callers).
+// counters plus kMaxVoxels index entries (32 MiB).
 constexpr long long kMaxVoxels = 1LL << 23;
-constexpr size_t kScratchBytes = 64 + 2 * (size_t)kMaxVoxels * sizeof(int);
+constexpr size_t kScratchBytes = 64 + (size_t)kMaxVoxels * sizeof(int);
 
 static __device__ __align__(256) unsigned char g_fill_scratch[kScratchBytes];
 
@@ -52,15 +52,15 @@ extern "C" int pct_regularize_device_noalloc(float *d_vol, int nx, int ny, int n
   // Compared factor by factor, so no product can overflow before the check.
   if (nx > kMaxVoxels || ny > kMaxVoxels / nx || nz > kMaxVoxels / ((long long)nx * ny))
     return PCT_ERR_TOO_LARGE;
-  static_assert(kScratchBytes >= 64 + 2 * (size_t)kMaxVoxels * sizeof(int), "scratch too small");
   void *scratch = nullptr;
+  if (pct::regularize_scratch_bytes((long long)nx * ny * nz) > kScratchBytes) return PCT_ERR_INTERNAL;
   if (scratch_address(&scratch) != cudaSuccess) {
     cudaGetLastError();
     return PCT_ERR_CUDA;
   }
   long long f = 0;
   int rounds = 0;
-  // launch_regularize zeroes the counter header itself before using the lists.
+  // launch_regularize zeroes the counter header itself before using the list.
   const cudaError_t e = pct::launch_regularize(d_vol, nx, ny, nz, nh, scratch,
                                                static_cast<cudaStream_t>(stream), &f, &rounds);
   if (e != cudaSuccess) {

@@ -1,10 +1,15 @@
 """The NaN fill where a median is itself NaN (both infinities in the middle), and where nothing can be
-filled: voxels, counts and time, against the rule in sweep order on the CPU."""
+filled: voxels, counts and time, against the rule in sweep order on the CPU; and the memory that its
+allocation-free form holds."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 import pseudoctimaging_b200 as pct
+from conftest import REPO
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +99,29 @@ def test_what_nothing_can_fill_ends_soon(shape, nh):
             times.append(a.elapsed_time(b))
     assert bool(vol.isnan().all())
     assert min(times[1:]) < 8.0, times
+
+
+NOALLOC = """
+import ctypes
+import torch
+import pseudoctimaging_b200 as pct
+n = 1 << 23
+v = torch.zeros(n, device="cuda")
+v[n // 2 + 64 * 128 + 64] = float("nan")
+with pct.Handle(0) as h:  # (the fill's own code is loaded)
+    h.regularize_device(torch.zeros(16 ** 3, device="cuda").data_ptr(), 16, 16, 16, 7)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+f = ctypes.c_int64(-1)
+st = pct.lib.pct_regularize_device_noalloc(v.data_ptr(), 128, 128, 512, 7, ctypes.byref(f), None)
+used = (free - torch.cuda.mem_get_info()[0]) / 2 ** 20
+print(st, f.value, int(v.isnan().sum()), used)
+"""
+
+
+def test_noalloc_form_holds_one_list():
+    """The largest volume it takes, in a process of its own: 32 MiB of index list."""
+    out = subprocess.run([sys.executable, "-c", NOALLOC], cwd=REPO, check=True, capture_output=True,
+                         text=True, timeout=120).stdout.split()
+    assert out[:3] == ["0", "1", "0"]
+    assert 30 <= float(out[3]) <= 40, out
