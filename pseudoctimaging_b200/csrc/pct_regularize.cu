@@ -111,11 +111,11 @@ __device__ __forceinline__ bool ready(const float *vol, int nx, int ny, int nz, 
 
 constexpr int kLooks = 256;  // passes over a warp's pending voxels per launch
 
-// The looks of one warp. It also ends them when no warp fills anything any more: it reads the fill
+// The looks of one warp with many voxels. It also ends them when no warp fills anything any more: it reads the fill
 // counter before every PER-th look and ends where two reads are equal and it filled nothing between
 // them (too early an end costs one more launch, about 15 us). Without the reads a volume that nothing
 // can fill went through all looks: 222x222x112, all NaN, 76 ms; 0.77 now, 0.88 with a launch per round.
-template <int PER, bool MANY>
+template <int PER>
 __device__ __forceinline__ void fill_looks(float *vol, int nx, int ny, int nz, int lo,
                                            const int *__restrict__ list, int n, int w, int nwarps,
                                            int lane, unsigned long long *fills,
@@ -134,7 +134,7 @@ __device__ __forceinline__ void fill_looks(float *vol, int nx, int ny, int nz, i
         const long long i = base + (long long)lane * nwarps;
         const int k = i < n ? list[i] : -1;
         unsigned todo = __ballot_sync(0xffffffffu, k >= 0 && isnan(*((volatile const float *)vol + max(k, 0))));
-        if (MANY && __popc(todo) > 2) {  // many voxels per warp: only the ready ones cost a warp's look
+        if (__popc(todo) > 2) {  // only the ready ones cost a warp's look
           const bool go = ((todo >> lane) & 1) && ready(vol, nx, ny, nz, lo, k);
           const unsigned to = __ballot_sync(0xffffffffu, go);
           left |= to != todo;
@@ -167,6 +167,36 @@ __device__ __forceinline__ void fill_looks(float *vol, int nx, int ny, int nz, i
   if (lane == 0 && nans) atomicAdd(nan_medians, (unsigned long long)nans);
 }
 
+// The same for at most 32 voxels per warp, which stay in its lanes' registers: a look is one round trip
+// to L2, and the counter is read after every sixteenth.
+__device__ __forceinline__ void fill_few(float *vol, int nx, int ny, int nz, int lo,
+                                         const int *__restrict__ list, int n, int w, int nwarps,
+                                         int lane, unsigned long long *fills,
+                                         unsigned long long *nan_medians) {
+  const long long i = w + (long long)lane * nwarps;
+  const int k = i < n ? list[i] : -1;
+  // (a launch after the first one finds some filled)
+  unsigned todo = __ballot_sync(0xffffffffu, k >= 0 && isnan(*((volatile const float *)vol + max(k, 0))));
+  unsigned long long seen = ~0ull;
+  for (int look = 0; todo && look < kLooks; ++look) {
+    unsigned filled = 0, nans = 0;
+    for (unsigned left = todo; left; left &= left - 1) {
+      const int j = __ffs(left) - 1;
+      const Look r = try_fill(vol, nx, ny, nz, lo, __shfl_sync(0xffffffffu, k, j), lane);
+      if (r == kWaits) continue;
+      todo &= ~(1u << j);
+      filled += r == kFilled;
+      nans += r == kNanMedian;
+    }
+    if (lane == 0 && filled) atomicAdd(fills, (unsigned long long)filled);
+    if (lane == 0 && nans) atomicAdd(nan_medians, (unsigned long long)nans);
+    if ((look & 15) != 15) continue;
+    const unsigned long long now = *(volatile unsigned long long *)fills;
+    if (__all_sync(0xffffffffu, now == seen)) break;
+    seen = now;
+  }
+}
+
 // A look takes 1 us with a voxel or two per warp and 300 us with a thousand, so the fewer there are,
 // the more looks lie between two reads of the counter (64x64x32, all NaN: 0.09 ms as with a launch per
 // round; 0.15 with eight looks between reads in the middle form, 1.8 without reads).
@@ -180,11 +210,11 @@ __global__ void __launch_bounds__(256) fill_kernel(float *vol, int nx, int ny, i
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (n <= 2 * nwarps)
-    fill_looks<16, false>(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
+    fill_few(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
   else if (n <= 64 * nwarps)
-    fill_looks<4, true>(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
+    fill_looks<4>(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
   else
-    fill_looks<1, true>(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
+    fill_looks<1>(vol, nx, ny, nz, lo, list, n, w, nwarps, lane, fills, nan_medians);
 }
 
 }  // namespace
