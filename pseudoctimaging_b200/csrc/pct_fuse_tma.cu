@@ -164,10 +164,13 @@ constexpr float kTileCost[5][4] = {{0.0185f, 0.0162f, 0.0146f, 0.0195f},
 
 // Expected time (us) of the volume's work items, `natl` atlases and 1 / splits of the window each:
 // rounds of the persistent grid, the last one cheaper when it leaves SMs with one CTA (one warp per
-// scheduler takes 0.61 of the time of two sharing it; 0.85 measured behind a full round), plus what
-// each item spends on its windows, taps and stores and, with partial sums, the combine. Within 10 %
-// of the measured times for 17 shapes from 48x40x30 to 222x222x112, every tile and split; the plan
-// chosen is 0..2 % behind the best of them on 14 of the 17, 11 % at worst.
+// scheduler takes 0.61 of the time of two sharing it; 0.85 behind several full rounds), plus what each
+// item spends on its windows, taps and stores and, with partial sums, the combine. Behind one full round
+// the remainder takes 0.44 of a round up to 110 of 296 slots (37 %) and a whole one from 112 on, and the
+// CTAs that take a second item pay its windows again: 7,000 plans of 380 shapes, where the rule for more
+// rounds put 1.08 rounds of 8 groups (40x23x93, 8 atlases, NH 3: 47 us) before half a round of 4 (39).
+// Of those shapes' best plans the chosen one is 1.2 % behind on average, 5 % or more on 36 of 380, 22 %
+// at worst (2.0 %, 54 and 40 % with that rule for one round too).
 double expected_us(const Geometry &g, const FusePlan &pl, int slots, double voxel_ns, int natl,
                    int splits, int groups) {
   const double rounds = (double)pl.tiles * groups / slots;
@@ -175,14 +178,18 @@ double expected_us(const Geometry &g, const FusePlan &pl, int slots, double voxe
   const double voxels = (double)kOutY * kWarps * pl.rx * 2 * pl.tz;
   const double round = 1e-3 * slots * voxels * voxel_ns * natl / splits;  // items of average length
   const double longest = round * splits * ((g.nh + splits - 1) / splits) / g.nh;
-  double t = 0.0;
-  if (full < 1.0)
+  double t = 0.0, items = std::max(1.0, rounds);  // items: of a CTA that takes the most of them
+  if (full < 1.0) {
     t = (rem <= 0.5 ? 0.61 : 1.0) * longest;
-  else if (rem > 0.0)
+  } else if (full == 1.0 && rem > 0.0) {
+    t = (rem < 0.365 ? 1.44 : 2.0) * round + longest - round;
+    items = 1.85;
+  } else if (rem > 0.0) {
     t = std::min((full + (rem <= 0.5 ? 0.85 : 1.0)) * round, (rounds + 0.4) * round) + longest - round;
-  else
+  } else {
     t = full * round + longest - round;
-  t += std::max(1.0, rounds) * (6.0 + 1.0 * natl);
+  }
+  t += items * (6.0 + 1.0 * natl);
   if (groups > 1) t += 2.5 + (double)g.ix * g.iy * g.iz * 16.0 * groups / 5e6;
   return t;
 }
