@@ -363,8 +363,8 @@ int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in
   *done = false;
   pct::OffsetRuns runs;
   const int k = h->learned_prior_k;
-  if (g.iy <= 0 || g.iz <= 0 || (long long)g.nz * g.nx * in.pitch >= (1LL << 31) - 1 ||
-      !pct::make_offset_runs(pct::learned::prior_offsets(k, g.hw), &runs))
+  // (the offsets are listed, a sort of the whole window, only once it is clear that they are needed)
+  if (k < 2 || g.iy <= 0 || g.iz <= 0 || (long long)g.nz * g.nx * in.pitch >= (1LL << 31) - 1)
     return PCT_OK;
   int st = ensure(h, h->err, 16);
   if (st) return st;
@@ -389,6 +389,7 @@ int launch_prior_tiles(pct_handle *h, const pct::Geometry &g, pct::SlabInputs in
                          static_cast<const float *>(h->label.ptr), pitch};
     note_capture(s, {&h->atlas, &h->label});
   }
+  if (!pct::make_offset_runs(pct::learned::prior_offsets(k, g.hw), &runs)) return PCT_OK;
   pct::FusePlan plan;
   if ((st = plan_fusion(h, g, 0, s, &plan, &runs))) return st;
   int *err = static_cast<int *>(h->err.ptr);
