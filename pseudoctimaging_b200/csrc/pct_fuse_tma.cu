@@ -385,7 +385,7 @@ void batch_plan_hw(const Geometry &g, FusePlan *pl, int *yb, int *za, int *zl) {
 template <int SET>
 cudaError_t batch_plan(int hw, const Geometry &g, FusePlan *pl, int *yb, int *za, int *zl) {
   *pl = FusePlan{};
-  pl->groups = pl->atlas_groups = pl->splits = 1;  // many subjects fill the grid; no partial sums
+  pl->groups = pl->atlas_groups = pl->splits = 1;  // (the batch's plan says how many: plan_batch)
   switch (hw) {
     case 5: batch_plan_hw<SET, 5>(g, pl, yb, za, zl); return cudaSuccess;
     case 4: batch_plan_hw<SET, 4>(g, pl, yb, za, zl); return cudaSuccess;
@@ -806,7 +806,7 @@ namespace {
 // One warp per row (grid-stride over rows), so that no element index is divided by the row
 // length; PAIRS copies 8-byte pairs (even ny and 8-byte aligned sources; the destinations' pitch
 // is a multiple of 4 floats). Rows past `rows` are the second stack's: one launch for both (two cost
-// 11 us of a 107 us call at 97x85x53, 3 atlases, NH 5; 102 us in one).
+// 4 us more of a call at 97x85x53, 3 atlases, NH 5: 106.6 us, 102.4 in one, timed in turn).
 template <bool PAIRS>
 __global__ void pitch_copy_kernel(const float *__restrict__ src0, float *__restrict__ dst0,
                                   const float *__restrict__ src1, float *__restrict__ dst1,

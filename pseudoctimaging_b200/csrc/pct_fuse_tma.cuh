@@ -671,10 +671,12 @@ __device__ __forceinline__ void pipe_drain(const Pipe &pp, unsigned long long ti
 }
 
 // Register tiles (x rows RX, z planes per half TZ, layout LY, CTAs per SM MB) by half window, in
-// sets the autotuner chooses between. Set 0 is the fastest measured shape per window on one B200
+// sets the autotuner chooses between. Set 0 was the fastest of sets 0 to 4 per window on one B200
 // (222x222x112, 10 atlases): y-pairs (3,4) for NH 7 and 11, y-pairs with the label ring (3,3)
-// for NH 9. Set 1 is the z-pair layout (3,4), set 2 the z-pair (3,3)/(4,2) tiles, set 3 y-pairs
-// with the label ring (3,4), set 4 y-pairs (2,3) at three CTAs per SM (168 registers).
+// for NH 9; of sets 5 to 7, which it chooses between by shape, the best takes 1 to 8 % less per voxel
+// (kTileCost).
+// Set 1 is the z-pair layout (3,4), set 2 the z-pair (3,3)/(4,2) tiles, set 3 y-pairs with the label
+// ring (3,4), set 4 y-pairs (2,3) at three CTAs per SM (168 registers).
 template <int SET, int HW> struct TileOf { static constexpr int RX = 3, TZ = 4, LY = 1, MB = 1; };
 template <> struct TileOf<0, 4> { static constexpr int RX = 3, TZ = 3, LY = 2, MB = 1; };
 template <> struct TileOf<0, 2> { static constexpr int RX = 3, TZ = 3, LY = 1, MB = 1; };
