@@ -615,17 +615,25 @@ int stage_pitched_slice(pct_handle *h, DevBuf &buf, float *stage_base, const flo
 // uploads (and repacks) the subject in parts, each part's work items starting as soon as it has
 // landed: the input MRI and the first atlas group in up to three plane ranges (the first holds
 // the planes read by just enough z-tiles to give every CTA of the grid an item, the second as
-// many z-tiles again, the third the rest), then one part per further group. The launches
+// many z-tiles again, the third the rest), then one part per further group, or several where a
+// group's stacks are small (kPartBytes: 43x47x34, 8 atlases, NH 3 0.27 ms pinned and 0.37 pageable, 0.35
+// and 0.44 with a part per group). With one group everything goes in three or four plane ranges of
+// equally many z-tiles, each of which fills half the grid or more; a range's outputs are complete once
+// its items are (222x222x112, 2 atlases, NH 7: 3.7 ms pinned, 5.2 in one piece; two ranges of a volume
+// with 272 tiles gain less than their copies cost, 0.99 ms against 0.76 for 71x215x34, 6 atlases, NH 3).
+// The launches
 // alternate between `s` and the handle's second compute stream, so that the last round of one
 // launch overlaps the first round of the next. With `host_out`, the last group runs in up to
 // three z-tile ranges as well (the last two as small as the first group's first), and the
 // handle's output stream combines and downloads each range's planes once its items and every
 // earlier launch are done, so that only the last range's combine and download follow the
 // fusion; without it, the group sums are combined into d_out on `s` at the end. Every stream
-// joins `s` before the call returns. Used when the plan has two or more atlas groups; returns
-// PCT_ERR_UNSUPPORTED (nothing enqueued) otherwise. `normalize` applies the label normalisation
+// joins `s` before the call returns. Returns PCT_ERR_UNSUPPORTED (nothing enqueued) where it does not
+// apply: one atlas whose window is split, and with one group also too few tiles for the ranges, inputs
+// below kOneGroupBytes, kernel timing and volumes that one range reads whole. `normalize` applies the label normalisation
 // to the CT stack on the device (the pipeline entry point). The items and the combine's group
 // order are those of the one-launch path, so the result is the same bit for bit.
+constexpr size_t kPartBytes = 2u << 20, kOneGroupBytes = 16u << 20;
 int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, const float *atlas,
                    const float *atlas_ct, float *d_out, double div, bool normalize,
                    float *host_out, cudaStream_t s) {
@@ -640,7 +648,14 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
                            (pitch != g.ny ? grow(h->stage, rows * g.ny * sizeof(float)) : 0),
                        s, &pl);
   if (st) return st;
-  if (pl.atlas_groups < 2 || h->wait_test_ns || ensure(h, h->atlas, rows * pitch * sizeof(float)) ||
+  const size_t plane = (size_t)g.nx * g.ny;
+  const bool one = pl.groups < 2;
+  const int ranges = one && pl.ctas > 0 ? std::min(4, 2 * pl.tiles / pl.ctas) : 0;
+  const bool applies = one ? !h->time_kernels && ranges > 2 &&
+                                 (2 * g.num + 1) * g.nz * plane * sizeof(float) >= kOneGroupBytes &&
+                                 pct::fuse_tma_planes_read(g, pl, (pl.tiles_z + ranges - 1) / ranges) < g.nz
+                           : pl.atlas_groups > 1;
+  if (!applies || h->wait_test_ns || ensure(h, h->atlas, rows * pitch * sizeof(float)) ||
       ensure(h, h->label, rows * pitch * sizeof(float)) || ensure(h, h->err, 16) ||
       (pitch != g.ny && try_ensure(h, h->stage, 2 * rows * g.ny * sizeof(float)))) {
     // (no room: the one-upload path needs half the staging, and takes the partial sums' place)
@@ -659,12 +674,28 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
   auto out_plane = [&](int tz) { return tz >= pl.tiles_z ? g.nz : g.lo + 2 * pl.tz * tz; };
   const int tiles_xy = pl.tiles_x * pl.tiles_y;
   const int first = std::min(pl.tiles_z, (pl.ctas + tiles_xy - 1) / tiles_xy);
-  if (pl.splits > 1) {  // a small volume: one part per atlas group, its items for the whole window
+  const size_t group_bytes = 2 * per * g.nz * plane * sizeof(float);
+  const int step = (int)std::max<size_t>(1, kPartBytes / std::max<size_t>(1, group_bytes));  // groups per part
+  if (one) {
+    int z0 = 0, t0 = 0;
+    for (int k = 1; k <= ranges && t0 < pl.tiles_z; ++k) {
+      int e = pl.tiles_z * k / ranges;
+      if (e <= t0) continue;
+      int z1 = pct::fuse_tma_planes_read(g, pl, e);
+      if (k == ranges || z1 >= g.nz) e = pl.tiles_z, z1 = g.nz;
+      parts.push_back(Part{true, 0, g.num, z0, z1, t0 * tiles_xy, e * tiles_xy,
+                           t0 == 0 ? 0 : out_plane(t0), host_out ? out_plane(e) : 0});
+      if (!host_out) parts.back().o0 = 0;
+      z0 = z1;
+      t0 = e;
+    }
+  } else if (pl.splits > 1) {  // a small volume: parts of atlas groups, their items for the whole window
     const int items = pl.splits * pl.tiles;
-    for (int grp = 0; grp < pl.atlas_groups; ++grp) {
-      const bool out_now = host_out && grp == pl.atlas_groups - 1;
-      parts.push_back(Part{grp == 0, grp * per, (grp + 1) * per, 0, g.nz, grp * items,
-                           (grp + 1) * items, 0, out_now ? g.nz : 0});
+    for (int grp = 0; grp < pl.atlas_groups; grp += step) {
+      const int end = std::min(grp + step, pl.atlas_groups);
+      const bool out_now = host_out && end == pl.atlas_groups;
+      parts.push_back(Part{grp == 0, grp * per, end * per, 0, g.nz, grp * items, end * items, 0,
+                           out_now ? g.nz : 0});
     }
   } else {
     // z-tile ends of the first group's leading parts; part k reads planes [0, planes_read(end))
@@ -679,9 +710,10 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
       t0 = e;
     }
     parts.push_back(Part{true, 0, per, z0, g.nz, t0 * tiles_xy, pl.tiles, 0, 0});
-    for (int grp = 1; grp < pl.groups - 1; ++grp)
-      parts.push_back(Part{false, grp * per, (grp + 1) * per, 0, g.nz, grp * pl.tiles,
-                           (grp + 1) * pl.tiles, 0, 0});
+    for (int grp = 1; grp < pl.groups - 1; grp += step) {
+      const int end = std::min(grp + step, pl.groups - 1);
+      parts.push_back(Part{false, grp * per, end * per, 0, g.nz, grp * pl.tiles, end * pl.tiles, 0, 0});
+    }
     const int last = pl.groups - 1;
     const int base = last * pl.tiles;
     if (!host_out) {
@@ -725,7 +757,6 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
   PCT_CUDA(h, cudaStreamWaitEvent(cs, h->pipe_ev[0], 0));
   PCT_CUDA(h, cudaStreamWaitEvent(lanes[1], h->pipe_ev[0], 0));
   if (os) PCT_CUDA(h, cudaStreamWaitEvent(os, h->pipe_ev[0], 0));
-  const size_t plane = (size_t)g.nx * g.ny;
   float *stage_mri = static_cast<float *>(h->stage.ptr);
   float *stage_ct = stage_mri ? stage_mri + rows * g.ny : nullptr;
   const pct::SlabInputs in{static_cast<const float *>(h->img.ptr),
@@ -756,7 +787,8 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     }
     const cudaStream_t ls = lanes[k & 1];
     PCT_CUDA(h, cudaStreamWaitEvent(ls, landed(last_upload), 0));
-    PCT_CUDA(h, pct::launch_fuse_tma_items(g, in, div, partial, err, pl, p.i0, p.i1, ls));
+    PCT_CUDA(h, pct::launch_fuse_tma_items(g, in, one ? d_out : nullptr, div, partial, err, pl,
+                                           p.i0, p.i1, ls));
     PCT_CUDA(h, cudaEventRecord(done(k), ls));
     return PCT_OK;
   };
@@ -766,8 +798,8 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
   auto run_output = [&](size_t k) -> int {
     const Part &p = parts[k];
     PCT_CUDA(h, cudaStreamWaitEvent(os, done(k), 0));
-    PCT_CUDA(h, cudaStreamWaitEvent(os, done(k - 1), 0));
-    PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, p.o0, p.o1, os));
+    if (!one && k > 0) PCT_CUDA(h, cudaStreamWaitEvent(os, done(k - 1), 0));
+    if (!one) PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, p.o0, p.o1, os));
     PCT_CUDA(h, download(h, host_out + p.o0 * plane, d_out + p.o0 * plane,
                          (size_t)(p.o1 - p.o0) * plane * sizeof(float), os));
     return PCT_OK;
@@ -789,7 +821,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
   st = PCT_OK;
   for (size_t k = 0; k < parts.size() && !st; ++k) st = run_part(k);
   h->stager.end();
-  for (size_t k = 1; k < parts.size() && !st; ++k)
+  for (size_t k = 0; k < parts.size() && !st; ++k)
     if (parts[k].o1 > parts[k].o0) st = run_output(k);
   // join (on failure too, so that nothing of this call is still running on the other streams
   // when the caller's next call reuses the buffers)
@@ -805,7 +837,7 @@ int fuse_pipelined(pct_handle *h, const pct::Geometry &g, const float *img, cons
     PCT_CUDA(h, cudaStreamWaitEvent(s, joined, 0));
   }
   if (st) return st;
-  if (!host_out)
+  if (!host_out && !one)
     PCT_CUDA(h, pct::launch_fuse_tma_combine(g, partial, pl, d_out, 0, g.nz, s));
   return PCT_OK;
 }

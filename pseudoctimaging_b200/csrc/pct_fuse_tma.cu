@@ -288,8 +288,8 @@ cudaError_t launch_hw(const Geometry &g, const SlabInputs &in, float *out, doubl
   if (whole) {
     item_begin = 0;
     item_end = pl.groups * pl.tiles;
-  } else if (pl.groups < 2 || item_begin >= item_end || item_end > pl.groups * pl.tiles) {
-    return cudaErrorInvalidValue;  // an item range needs partial sums and a later combine
+  } else if ((pl.groups < 2 && !out) || item_begin >= item_end || item_end > pl.groups * pl.tiles) {
+    return cudaErrorInvalidValue;
   }
   cudaError_t e;
   CUtensorMap tmA, tmL;
@@ -786,13 +786,13 @@ cudaError_t launch_fuse_tma(const Geometry &g, const SlabInputs &in, float *out,
   return launch_any(g, in, out, div, partial, err, wt, plan, -1, -1, stream);
 }
 
-cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, double div,
+cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, float *out, double div,
                                   float *partial, int *err, const FusePlan &plan, int item_begin,
                                   int item_end, cudaStream_t stream) {
   if (g.ix <= 0 || g.iy <= 0 || g.iz <= 0) return cudaSuccess;
   if (item_begin < 0) return cudaErrorInvalidValue;
   const LaunchHooks wt{0, nullptr, nullptr};
-  return launch_any(g, in, nullptr, div, partial, err, wt, plan, item_begin, item_end, stream);
+  return launch_any(g, in, out, div, partial, err, wt, plan, item_begin, item_end, stream);
 }
 
 cudaError_t launch_fuse_tma_combine(const Geometry &g, const float *partial, const FusePlan &plan,

@@ -66,11 +66,10 @@ cudaError_t fuse_tma_plan(const Geometry &g, int set, size_t partial_limit, Fuse
 cudaError_t launch_fuse_tma(const Geometry &g, const SlabInputs &in, float *out, double div,
                             float *partial, int *err, const LaunchHooks &wt, const FusePlan &plan,
                             cudaStream_t stream);
-// Pipelined form of the same (plans with 2 or more groups only): the work items
-// [item_begin, item_end) into the partial sums; launch_fuse_tma_combine adds the groups into out
-// once every item has run. Lets the host start on the first planes of the first group while the
-// rest is uploaded.
-cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, double div,
+// Pipelined form of the same: the work items [item_begin, item_end), with one group into out, with
+// more into the partial sums; launch_fuse_tma_combine then adds the groups into out once every item
+// has run. Lets the host start on the first planes while the rest is uploaded.
+cudaError_t launch_fuse_tma_items(const Geometry &g, const SlabInputs &in, float *out, double div,
                                   float *partial, int *err, const FusePlan &plan, int item_begin,
                                   int item_end, cudaStream_t stream);
 // Planes [0, n) of the input and atlas volumes that the items of z-tiles [0, ztiles) read.
